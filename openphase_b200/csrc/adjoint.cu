@@ -879,7 +879,8 @@ __global__ void adjoint_bulk_kernel(const __grid_constant__ StepParams p, const 
 
 // Wide voxels whose list has N fields, from the classify kernel's work records (the lists, values
 // and Laplacians the forward step used; own fields are the leading nonzero values).
-template <class R, int N, int KS>
+// (N <= kListCap fields always fit the state's slots: the core's record never overflows.)
+template <class R, int N>
 __global__ void __launch_bounds__(128) adjoint_list_kernel(const __grid_constant__ StepParams p, const StepArrays a,
                                                             const AdjArrays aa, int nslices)
 {
@@ -915,7 +916,7 @@ __global__ void __launch_bounds__(128) adjoint_list_kernel(const __grid_constant
             own = own && val[k] != 0.0;
             c += own ? 1 : 0;
         }
-        adjoint_core<N, KS, R>(p, a, aa, v, flag, N, c, g, val, lap, 0u);
+        adjoint_core<N, kListCap, R>(p, a, aa, v, flag, N, c, g, val, lap, 0u);
     }
 }
 
@@ -975,14 +976,14 @@ __device__ __forceinline__ double gather_global(const StepParams& p, const AdjAr
     return l;
 }
 
-template <int KS, int NS>
+template <int NS>
 __global__ void __launch_bounds__(kTileZ * kTileTY)
 adjoint_gather_kernel(const __grid_constant__ StepParams p, const StepArrays la, const uint8_t* __restrict__ cnt,
                       const int16_t* __restrict__ idx, const AdjArrays aa, double* __restrict__ lam0, int xchunk)
 {
     constexpr int TY = kTileTY;
     using Geo = TileGeom<TY>;
-    using Smem = TileSmem<double, KS, TY>;
+    using Smem = TileSmem<double, TY>;
     constexpr int NT = Geo::NT;
     constexpr int kC = Geo::kCols;
     constexpr int kSlots = WindowSlots<double>::value;
@@ -1061,17 +1062,17 @@ adjoint_gather_kernel(const __grid_constant__ StepParams p, const StepArrays la,
     }
 }
 
-template <int KS, int NS>
+template <int NS>
 static int launch_gather_ns(const StepParams& p, const StepArrays& a, const AdjArrays& aa, double* lam0, cudaStream_t s)
 {
-    using Smem = TileSmem<double, KS, kTileTY>;
+    using Smem = TileSmem<double, kTileTY>;
     int xchunk = 0, gz = 0, gy = 0, gx = 0;
     tiled_geometry(p.nx, p.ny, p.nz, &xchunk, &gz, &gy, &gx);
     StepArrays la = a;   // the plane loader reads the lists of the Laplacian adjoints
     la.cnt_in = aa.lcnt;
     la.idx_in = aa.lidx;
     la.val_in = aa.llam;
-    auto kern = adjoint_gather_kernel<KS, NS>;
+    auto kern = adjoint_gather_kernel<NS>;
     const size_t smem = sizeof(Smem);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
@@ -1079,11 +1080,10 @@ static int launch_gather_ns(const StepParams& p, const StepArrays& a, const AdjA
     return (int)cudaGetLastError();
 }
 
-template <int KS>
 static int launch_gather(const StepParams& p, const StepArrays& a, const AdjArrays& aa, double* lam0, cudaStream_t s)
 {
-    if (p.ns == 27) return launch_gather_ns<KS, 27>(p, a, aa, lam0, s);
-    if (p.ns == 7) return launch_gather_ns<KS, 7>(p, a, aa, lam0, s);
+    if (p.ns == 27) return launch_gather_ns<27>(p, a, aa, lam0, s);
+    if (p.ns == 7) return launch_gather_ns<7>(p, a, aa, lam0, s);
     return -1;
 }
 
@@ -1113,57 +1113,46 @@ int launch_tlm_step(const StepParams& p, const StepArrays& a, const AdjArrays& a
 
 constexpr int kAdjListBlocks = 148 * 32;   // blocks of each per-length adjoint kernel
 
-// The worklist kernel (few voxels, each a long serial chain) runs on the side stream, launched
-// first, so that it overlaps the list-length kernels instead of adding its latency after them.
+// The per-length kernels, the worklist kernel (few voxels, each a long serial chain: its own stream)
+// and the bulk kernel write disjoint voxels and run beside each other; each is a latency chain on
+// small grids (56 x 60 x 50, FP64: 51, 109, 136, 115, 130, 172, 228 us for N = 2..8, worklist
+// 533 us).
 template <class R, int KS>
-static void adjoint_kernels(const StepParams& p, const StepArrays& a, const AdjArrays& aa, int nblocks, cudaStream_t s,
-                            cudaStream_t side)
+static void adjoint_kernels(const StepParams& p, const StepArrays& a, const AdjArrays& aa, int nblocks,
+                            const SideFork& fork)
 {
-    adjoint_worklist_kernel<R, KS><<<148 * 4, 64, 0, side>>>(p, a, aa);
-    adjoint_list_kernel<R, 2, KS><<<kAdjListBlocks, 128, 0, s>>>(p, a, aa, nblocks);
-    adjoint_list_kernel<R, 3, KS><<<kAdjListBlocks, 128, 0, s>>>(p, a, aa, nblocks);
-    adjoint_list_kernel<R, 4, KS><<<kAdjListBlocks, 128, 0, s>>>(p, a, aa, nblocks);
-    adjoint_list_kernel<R, 5, KS><<<kAdjListBlocks, 128, 0, s>>>(p, a, aa, nblocks);
-    adjoint_list_kernel<R, 6, KS><<<kAdjListBlocks, 128, 0, s>>>(p, a, aa, nblocks);
-    adjoint_list_kernel<R, 7, KS><<<kAdjListBlocks, 128, 0, s>>>(p, a, aa, nblocks);
-    adjoint_list_kernel<R, 8, KS><<<kAdjListBlocks, 128, 0, s>>>(p, a, aa, nblocks);
+    const cudaStream_t s = fork.main;
+    adjoint_worklist_kernel<R, KS><<<148 * 4, 64, 0, fork.on(2)>>>(p, a, aa);
+    adjoint_list_kernel<R, 8><<<kAdjListBlocks, 128, 0, fork.on(0)>>>(p, a, aa, nblocks);
+    adjoint_list_kernel<R, 7><<<kAdjListBlocks, 128, 0, fork.on(1)>>>(p, a, aa, nblocks);
+    adjoint_list_kernel<R, 6><<<kAdjListBlocks, 128, 0, s>>>(p, a, aa, nblocks);
+    adjoint_list_kernel<R, 5><<<kAdjListBlocks, 128, 0, fork.on(3)>>>(p, a, aa, nblocks);
+    adjoint_list_kernel<R, 4><<<kAdjListBlocks, 128, 0, s>>>(p, a, aa, nblocks);
+    adjoint_list_kernel<R, 3><<<kAdjListBlocks, 128, 0, fork.on(3)>>>(p, a, aa, nblocks);
+    adjoint_list_kernel<R, 2><<<kAdjListBlocks, 128, 0, fork.on(1)>>>(p, a, aa, nblocks);
+    adjoint_bulk_kernel<<<grid_of(p.n, 256), 256, 0, s>>>(p, a.cnt_in, aa);
 }
 
 int launch_adjoint_step(const StepParams& p, const StepArrays& a, const AdjArrays& aa, int k_slots, bool fp32,
-                        int nblocks, double* lam0, void* stream, const AdjStreams& fork)
+                        int nblocks, double* lam0, void* stream, const SideStreams& side)
 {
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    cudaStream_t side = fork.side ? static_cast<cudaStream_t>(fork.side) : s;
-    adjoint_bulk_kernel<<<grid_of(p.n, 256), 256, 0, s>>>(p, a.cnt_in, aa);
-    cudaError_t e;
-    if (side != s)
-    {
-        if ((e = cudaEventRecord(static_cast<cudaEvent_t>(fork.ev_fork), s)) != cudaSuccess) return (int)e;
-        if ((e = cudaStreamWaitEvent(side, static_cast<cudaEvent_t>(fork.ev_fork), 0)) != cudaSuccess) return (int)e;
-    }
+    const SideFork fork(&side, s);
+    bool known = true;
     switch (k_slots * 2 + (fp32 ? 1 : 0))
     {
-        case 16: adjoint_kernels<double, 8>(p, a, aa, nblocks, s, side); break;
-        case 17: adjoint_kernels<float, 8>(p, a, aa, nblocks, s, side); break;
-        case 24: adjoint_kernels<double, 12>(p, a, aa, nblocks, s, side); break;
-        case 25: adjoint_kernels<float, 12>(p, a, aa, nblocks, s, side); break;
-        case 32: adjoint_kernels<double, 16>(p, a, aa, nblocks, s, side); break;
-        case 33: adjoint_kernels<float, 16>(p, a, aa, nblocks, s, side); break;
-        default: return -1;
+        case 16: adjoint_kernels<double, 8>(p, a, aa, nblocks, fork); break;
+        case 17: adjoint_kernels<float, 8>(p, a, aa, nblocks, fork); break;
+        case 24: adjoint_kernels<double, 12>(p, a, aa, nblocks, fork); break;
+        case 25: adjoint_kernels<float, 12>(p, a, aa, nblocks, fork); break;
+        case 32: adjoint_kernels<double, 16>(p, a, aa, nblocks, fork); break;
+        case 33: adjoint_kernels<float, 16>(p, a, aa, nblocks, fork); break;
+        default: known = false; break;
     }
-    if (side != s)
-    {
-        if ((e = cudaEventRecord(static_cast<cudaEvent_t>(fork.ev_join), side)) != cudaSuccess) return (int)e;
-        if ((e = cudaStreamWaitEvent(s, static_cast<cudaEvent_t>(fork.ev_join), 0)) != cudaSuccess) return (int)e;
-    }
-    int rc = -1;
-    switch (k_slots)
-    {
-        case 8:  rc = launch_gather<8>(p, a, aa, lam0, s); break;
-        case 12: rc = launch_gather<12>(p, a, aa, lam0, s); break;
-        case 16: rc = launch_gather<16>(p, a, aa, lam0, s); break;
-        default: return -1;
-    }
+    const cudaError_t e = fork.join();
+    if (!known) return -1;
+    if (e != cudaSuccess) return (int)e;
+    const int rc = launch_gather(p, a, aa, lam0, s);
     if (rc != 0) return rc;
     return (int)cudaGetLastError();
 }

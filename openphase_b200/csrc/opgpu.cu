@@ -25,9 +25,7 @@ struct opgpu_ctx {
     opgpu_grid grid{};
     int device = 0;
     cudaStream_t stream = nullptr;
-    void* adj_side = nullptr;            // adjoint: side stream of the worklist kernel, fork / join events
-    void* adj_fork = nullptr;
-    void* adj_join = nullptr;
+    SideStreams side;                    // independent kernels of a step run beside each other on these
     std::string err;
     long long n = 0;
     int K = 8;
@@ -551,6 +549,19 @@ extern "C" uint32_t opgpu_create(const opgpu_grid* grid, opgpu_ctx** out)
     auto bail = [&](uint32_t code) { opgpu_destroy(ctx); return code; };
     if (cudaSetDevice(ctx->device) != cudaSuccess) return bail(OPGPU_E_CUDA);
     if (cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess) return bail(OPGPU_E_CUDA);
+    {
+        cudaEvent_t ev;
+        if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) return bail(OPGPU_E_CUDA);
+        ctx->side.fork = ev;
+        for (int k = 0; k < kSideStreams; k++)
+        {
+            cudaStream_t st;
+            if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) return bail(OPGPU_E_CUDA);
+            ctx->side.stream[k] = st;
+            if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) return bail(OPGPU_E_CUDA);
+            ctx->side.join[k] = ev;
+        }
+    }
     for (int b = 0; b < 2; b++)
     {
         if (dalloc(&ctx->cnt[b], (size_t)ctx->n) != cudaSuccess) return bail(OPGPU_E_CUDA);
@@ -623,9 +634,12 @@ extern "C" uint32_t opgpu_destroy(opgpu_ctx* ctx)
     dfree(ctx->d_lam_local); dfree(ctx->d_lcnt); dfree(ctx->d_lidx); dfree(ctx->d_llam);
     dfree(ctx->d_gsig); dfree(ctx->d_gmu); dfree(ctx->d_gdg);
     dfree(ctx->d_tsig); dfree(ctx->d_tmu); dfree(ctx->d_tdg); dfree(ctx->d_tvol);
-    if (ctx->adj_side) cudaStreamDestroy(static_cast<cudaStream_t>(ctx->adj_side));
-    if (ctx->adj_fork) cudaEventDestroy(static_cast<cudaEvent_t>(ctx->adj_fork));
-    if (ctx->adj_join) cudaEventDestroy(static_cast<cudaEvent_t>(ctx->adj_join));
+    for (int k = 0; k < kSideStreams; k++)
+    {
+        if (ctx->side.stream[k]) cudaStreamDestroy(static_cast<cudaStream_t>(ctx->side.stream[k]));
+        if (ctx->side.join[k]) cudaEventDestroy(static_cast<cudaEvent_t>(ctx->side.join[k]));
+    }
+    if (ctx->side.fork) cudaEventDestroy(static_cast<cudaEvent_t>(ctx->side.fork));
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
     return OPGPU_OK;
@@ -1225,6 +1239,7 @@ static uint32_t enqueue_steps(opgpu_ctx* ctx, double dt, int nsteps, bool partia
         a.bucket = ctx->d_bucket; a.bucket_count = ctx->d_bucket_count; a.bucket_off = ctx->d_bucket_off;
         a.bucket_cap = ctx->bucket_cap; a.slice = ctx->slice;
         LaunchInfo info;
+        info.side = &ctx->side;
         if (ctx->timing)
         {
             if (ctx->ev_pool.size() < 3 * (ctx->ev_used + 1))
@@ -1556,17 +1571,6 @@ uint32_t ensure_adjoint(opgpu_ctx* ctx)
     CK(dalloc(&ctx->d_gsig, G * G));
     CK(dalloc(&ctx->d_gmu, G * G));
     CK(dalloc(&ctx->d_gdg, G));
-    if (!ctx->adj_side)
-    {
-        cudaStream_t side;
-        cudaEvent_t ef, ej;
-        CK(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
-        ctx->adj_side = side;
-        CK(cudaEventCreateWithFlags(&ef, cudaEventDisableTiming));
-        ctx->adj_fork = ef;
-        CK(cudaEventCreateWithFlags(&ej, cudaEventDisableTiming));
-        ctx->adj_join = ej;
-    }
     ctx->adjoint_ready = true;
     return OPGPU_OK;
 }
@@ -1701,14 +1705,13 @@ extern "C" uint32_t opgpu_adjoint_step(opgpu_ctx* ctx, int32_t slot, double dt)
     a.wl = ctx->d_wl; a.wl_slice = ctx->wl_slice;
     a.bucket = ctx->d_bucket; a.bucket_count = ctx->d_bucket_count; a.bucket_off = ctx->d_bucket_off;
     a.bucket_cap = ctx->bucket_cap; a.slice = ctx->slice;
-    const int nblocks = ctx->fp32 ? launch_classify_f32(sp, a, ctx->K, ctx->stream)
-                                  : launch_classify_f64(sp, a, ctx->K, ctx->stream);
+    const int nblocks = ctx->fp32 ? launch_classify_f32(sp, a, ctx->stream)
+                                  : launch_classify_f64(sp, a, ctx->stream);
     if (nblocks < 0) return fail(ctx, OPGPU_E_CUDA, "opgpu_adjoint_step: classify launch");
     CK(cudaMemsetAsync(ctx->d_vol_acc, 0, (size_t)ctx->G * sizeof(double), ctx->stream));
     CK(cudaMemsetAsync(ctx->d_counters, 0, 3 * sizeof(unsigned long long), ctx->stream));   // wide, entries in/out
     CK(cudaMemsetAsync(ctx->d_counters + kCntCrowdedLast, 0, sizeof(unsigned long long), ctx->stream));
-    const AdjStreams fork{ctx->adj_side, ctx->adj_fork, ctx->adj_join};
-    if (launch_adjoint_step(sp, a, aa, ctx->K, ctx->fp32 != 0, nblocks, lam0, ctx->stream, fork))
+    if (launch_adjoint_step(sp, a, aa, ctx->K, ctx->fp32 != 0, nblocks, lam0, ctx->stream, ctx->side))
         return fail(ctx, OPGPU_E_CUDA, "opgpu_adjoint_step: launch");
     ctx->kernel_launches += 12;
     ctx->lam_cur = 1 - ctx->lam_cur;

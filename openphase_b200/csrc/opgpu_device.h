@@ -174,10 +174,20 @@ inline void tiled_geometry(int nx, int ny, int nz, int* xchunk, int* gz, int* gy
 
 enum { kVariantTiled = 0, kVariantGeneric = 1 };
 
+// Side streams of a context: independent kernels of one step run beside each other between a fork
+// from and a join into the context's stream.
+constexpr int kSideStreams = 4;
+struct SideStreams {
+    void* stream[kSideStreams] = {};   // cudaStream_t
+    void* fork = nullptr;              // cudaEvent_t
+    void* join[kSideStreams] = {};     // cudaEvent_t
+};
+
 // Filled by the launchers: kernels launched, and an event recorded after the classify kernel
 // (when `after_classify` is not null) so the caller can time it separately.
 struct LaunchInfo {
     void* after_classify = nullptr;   // cudaEvent_t
+    const SideStreams* side = nullptr;   // null: every kernel on the context's stream
     int kernels = 0;
 };
 
@@ -188,8 +198,8 @@ int launch_step_f64(const StepParams& p, const StepArrays& a, int k_slots, int v
 int launch_step_f32(const StepParams& p, const StepArrays& a, int k_slots, int variant, void* stream,
                     LaunchInfo* info);
 // The classify kernel of the tiled step alone; returns the number of classify blocks or < 0.
-int launch_classify_f64(const StepParams& p, const StepArrays& a, int k_slots, void* stream);
-int launch_classify_f32(const StepParams& p, const StepArrays& a, int k_slots, void* stream);
+int launch_classify_f64(const StepParams& p, const StepArrays& a, void* stream);
+int launch_classify_f32(const StepParams& p, const StepArrays& a, void* stream);
 // Driving-force averaging of a state (average.cu): launch_average_scan counts the pair slots of
 // every voxel, scans them into aa.off and writes their total to d_total; launch_average then writes
 // aa.tmp and aa.lim.  average_scan_bytes gives the scan's scratch bytes for n voxels.

@@ -10,9 +10,9 @@ int launch_step_f64(const StepParams& p, const StepArrays& a, int k_slots, int v
     return launch_step<double>(p, a, k_slots, variant, stream, info);
 }
 
-int launch_classify_f64(const StepParams& p, const StepArrays& a, int k_slots, void* stream)
+int launch_classify_f64(const StepParams& p, const StepArrays& a, void* stream)
 {
-    return launch_classify<double>(p, a, k_slots, stream);
+    return launch_classify<double>(p, a, stream);
 }
 
 // Grain volumes of the window planes of a state (slab decomposition: before the first step).

@@ -67,7 +67,7 @@ struct TileGeom {
     static constexpr int NT = kTileZ * TY;
 };
 
-template <class R, int KS, int TY>
+template <class R, int TY>
 struct TileSmem {
     using Geo = TileGeom<TY>;
     static constexpr int kSlots = WindowSlots<R>::value;
@@ -193,8 +193,8 @@ struct PlaneLoad {
 //                 the ring position held before
 // cr holds the plane's counts on entry (prefetched) and the next plane's counts after plane_fill.
 // Invariant of the dense planes: dense[k][rs][r] != 0 only if bit k of word[rs][r] is set.
-template <class R, int KS, int TY>
-__device__ __forceinline__ bool plane_scan(const StepParams& p, const StepArrays& a, TileSmem<R, KS, TY>& S,
+template <class R, int TY>
+__device__ __forceinline__ bool plane_scan(const StepParams& p, const StepArrays& a, TileSmem<R, TY>& S,
                                            int xp, int wpos, int y0, int z0, int t,
                                            const int (&cr)[PlaneRegs<TY>::kPer], PlaneLoad<R, TY>& L)
 {
@@ -252,8 +252,8 @@ __device__ __forceinline__ bool plane_scan(const StepParams& p, const StepArrays
     return added;
 }
 
-template <class R, int KS, int TY>
-__device__ __forceinline__ void plane_assign(TileSmem<R, KS, TY>& S, int wpos, int t)
+template <class R, int TY>
+__device__ __forceinline__ void plane_assign(TileSmem<R, TY>& S, int wpos, int t)
 {
     // warp 0 hands free slots (grain gone from the window) to the pending grains; lane 0 keeps
     // the grain -> slot hash in step
@@ -293,8 +293,8 @@ __device__ __forceinline__ void plane_assign(TileSmem<R, KS, TY>& S, int wpos, i
     }
 }
 
-template <class R, int KS, int TY>
-__device__ __forceinline__ void plane_fill(const StepParams& p, const StepArrays& a, TileSmem<R, KS, TY>& S,
+template <class R, int TY>
+__device__ __forceinline__ void plane_fill(const StepParams& p, const StepArrays& a, TileSmem<R, TY>& S,
                                            int rs, int xp, int y0, int z0, int t, int (&cr)[PlaneRegs<TY>::kPer],
                                            const PlaneLoad<R, TY>& L)
 {
@@ -339,8 +339,8 @@ __device__ __forceinline__ void plane_fill(const StepParams& p, const StepArrays
 }
 
 // The three passes with their barriers, for kernels that do not overlap plane_scan with other work.
-template <class R, int KS, int TY>
-__device__ __forceinline__ void load_plane(const StepParams& p, const StepArrays& a, TileSmem<R, KS, TY>& S,
+template <class R, int TY>
+__device__ __forceinline__ void load_plane(const StepParams& p, const StepArrays& a, TileSmem<R, TY>& S,
                                            int rs, int xp, int wpos, int y0, int z0, int t,
                                            int (&cr)[PlaneRegs<TY>::kPer])
 {
@@ -362,8 +362,8 @@ template <int NS>
 __device__ __forceinline__ constexpr int stencil_dz(int q) { return NS == 27 ? q % 3 - 1 : (q == 2 ? -1 : (q == 4 ? 1 : 0)); }
 
 // New grains of neighbour record (pl, r): append them (4-bit slot ids) in the record's entry order.
-template <class R, int KS, int TY>
-__device__ __forceinline__ void append_fresh(const TileSmem<R, KS, TY>& S, int pl, int r, uint32_t fresh,
+template <class R, int TY>
+__device__ __forceinline__ void append_fresh(const TileSmem<R, TY>& S, int pl, int r, uint32_t fresh,
                                              uint64_t& ls, int& n, bool& over)
 {
     const int cu = S.cntr[pl][r];
@@ -379,12 +379,12 @@ __device__ __forceinline__ void append_fresh(const TileSmem<R, KS, TY>& S, int p
     }
 }
 
-template <class R, int KS, int TY, int NS>
+template <class R, int TY, int NS>
 __global__ void __launch_bounds__(kTileZ * TY)
 tile_classify_kernel(const __grid_constant__ StepParams p, const StepArrays a, int xchunk)
 {
     using Geo = TileGeom<TY>;
-    using Smem = TileSmem<R, KS, TY>;
+    using Smem = TileSmem<R, TY>;
     constexpr int NT = Geo::NT;
     constexpr int kC = Geo::kCols;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -619,7 +619,9 @@ constexpr int kVolCache = 4;       // per-thread grain-volume cache of the compu
 // order is that of list_step.  The entries of length N from all classify slices form one index
 // range (bucket_off); each CUDA block takes an equal contiguous part of it, its warps 32
 // consecutive entries at a time, so that no warp idles while another drains a long slice.
-template <class R, int N, int KS>
+//
+// N <= kListCap <= the stored fields per voxel, so a new record always fits.
+template <class R, int N>
 __global__ void __launch_bounds__(128) list_compute_kernel(const __grid_constant__ StepParams p, const StepArrays a,
                                                            int nslices)
 {
@@ -901,7 +903,7 @@ __global__ void __launch_bounds__(128) list_compute_kernel(const __grid_constant
 #pragma unroll
         for (int i = 0; i < N; i++)
         {
-            if (keep[i] && pos < KS)
+            if (keep[i])
             {
                 const R w = (m > 1) ? (R)(vd[i] * norm) : R(1);
                 if (!isfinite((double)w)) st |= kStNonFinite;
@@ -929,7 +931,6 @@ __global__ void __launch_bounds__(128) list_compute_kernel(const __grid_constant
             }
         }
         if (m == 0) st |= kStEmptyVoxel;
-        if (m > KS) st |= kStOverflowK;
         a.cnt_out[v] = (uint8_t)pos;
         eout += pos;
         }
@@ -940,15 +941,67 @@ __global__ void __launch_bounds__(128) list_compute_kernel(const __grid_constant
     flush_block(a, 0u, 0u, eout, st, s_cnt, s_key, s_sum, kTileVolSlots, t, blockDim.x);
 }
 
+// Fork of the side streams from a context's stream, and their join into it.  join() is called on
+// every path that launched on them, so that no work of a step outlives the step's place in the
+// context's stream.
+struct SideFork {
+    const SideStreams* side;
+    cudaStream_t main;
+    cudaError_t err = cudaSuccess;
+
+    SideFork(const SideStreams* side_, cudaStream_t s) : side(side_), main(s)
+    {
+        if (!side) return;
+        err = cudaEventRecord(static_cast<cudaEvent_t>(side->fork), main);
+        for (int k = 0; k < kSideStreams && err == cudaSuccess; k++)
+            err = cudaStreamWaitEvent(on(k), static_cast<cudaEvent_t>(side->fork), 0);
+        if (err != cudaSuccess) side = nullptr;   // nothing forked is used
+    }
+    cudaStream_t on(int k) const { return side ? static_cast<cudaStream_t>(side->stream[k]) : main; }
+    cudaError_t join() const
+    {
+        if (!side) return err;
+        cudaError_t e = cudaSuccess;
+        for (int k = 0; k < kSideStreams; k++)
+        {
+            cudaError_t q = cudaEventRecord(static_cast<cudaEvent_t>(side->join[k]), on(k));
+            if (q == cudaSuccess) q = cudaStreamWaitEvent(main, static_cast<cudaEvent_t>(side->join[k]), 0);
+            if (e == cudaSuccess) e = q;
+        }
+        return e;
+    }
+};
+
+// The per-length kernels and the general path write disjoint voxels, so they run beside each other.
+// On small grids each is a chain of dependent arithmetic and instruction fetches whose length hardly
+// depends on the entry count (64^3, FP64: 17, 19, 26, 34, 54, 77, 115 us for N = 2..8), so the chains
+// are dealt out to streams of about equal length, the longest alone.  On large grids every kernel fills
+// the device and only the tails overlap, while the mixed resident blocks cost cache hits.  Step, one
+// stream -> side streams (FP64, us): 64^3 337 -> 192, 128^3 1024 -> 794, 192^3 2520 -> 2355, 224^3
+// 3749 -> 3690, 256^3 5465 -> 5600: the line lies between the last two.
+constexpr long long kSideVoxels = 12000000;
+template <class R>
+void launch_lists(const StepParams& p, const StepArrays& a, int cb, int nblocks, const SideFork& fork)
+{
+    const cudaStream_t s = fork.main;
+    list_compute_kernel<R, 8><<<cb, 128, 0, fork.on(0)>>>(p, a, nblocks);
+    list_compute_kernel<R, 7><<<cb, 128, 0, fork.on(1)>>>(p, a, nblocks);
+    list_compute_kernel<R, 6><<<cb, 128, 0, s>>>(p, a, nblocks);
+    list_compute_kernel<R, 5><<<cb, 128, 0, fork.on(3)>>>(p, a, nblocks);
+    list_compute_kernel<R, 4><<<cb, 128, 0, s>>>(p, a, nblocks);
+    list_compute_kernel<R, 3><<<cb, 128, 0, fork.on(3)>>>(p, a, nblocks);
+    list_compute_kernel<R, 2><<<cb, 128, 0, fork.on(1)>>>(p, a, nblocks);
+}
+
 template <class R, int KS, int KL, int NS>
 int launch_tiled_ns(const StepParams& p, const StepArrays& a, void* stream, LaunchInfo* info)
 {
-    using Smem = TileSmem<R, KS, kTileTY>;
+    using Smem = TileSmem<R, kTileTY>;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     int xchunk = 0, gz = 0, gy = 0, gx = 0;
     tiled_geometry(p.nx, p.ny, p.nz, &xchunk, &gz, &gy, &gx);
     const int nblocks = gz * gy * gx;
-    auto kern = tile_classify_kernel<R, KS, kTileTY, NS>;
+    auto kern = tile_classify_kernel<R, kTileTY, NS>;
     const size_t smem = sizeof(Smem);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
@@ -962,21 +1015,14 @@ int launch_tiled_ns(const StepParams& p, const StepArrays& a, void* stream, Laun
     }
     bucket_scan_kernel<<<kListCap - 1, 1024, 0, s>>>(a, nblocks);
     const int cb = compute_blocks(p.n);
-    list_compute_kernel<R, 2, KS><<<cb, 128, 0, s>>>(p, a, nblocks);
-    list_compute_kernel<R, 3, KS><<<cb, 128, 0, s>>>(p, a, nblocks);
-    list_compute_kernel<R, 4, KS><<<cb, 128, 0, s>>>(p, a, nblocks);
-    list_compute_kernel<R, 5, KS><<<cb, 128, 0, s>>>(p, a, nblocks);
-    list_compute_kernel<R, 6, KS><<<cb, 128, 0, s>>>(p, a, nblocks);
-    list_compute_kernel<R, 7, KS><<<cb, 128, 0, s>>>(p, a, nblocks);
-    list_compute_kernel<R, 8, KS><<<cb, 128, 0, s>>>(p, a, nblocks);
-    // general path: one warp per voxel of the worklist
-    {
-        auto gk = warp_general_kernel<R, KS, KL>;
-        const size_t wsm = 4 * sizeof(WarpScratch<R, KL>);
-        e = cudaFuncSetAttribute(gk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wsm);
-        if (e != cudaSuccess) return (int)e;
-        gk<<<148 * 4, 128, wsm, s>>>(p, a);
-    }
+    auto gk = warp_general_kernel<R, KS, KL>;
+    const size_t wsm = 4 * sizeof(WarpScratch<R, KL>);
+    e = cudaFuncSetAttribute(gk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wsm);
+    if (e != cudaSuccess) return (int)e;
+    const SideFork fork(info && p.n <= kSideVoxels ? info->side : nullptr, s);
+    gk<<<148 * 4, 128, wsm, fork.on(2)>>>(p, a);
+    launch_lists<R>(p, a, cb, nblocks, fork);
+    if ((e = fork.join()) != cudaSuccess) return (int)e;
     if (info) info->kernels += 10;
     return (int)cudaGetLastError();
 }
@@ -984,14 +1030,14 @@ int launch_tiled_ns(const StepParams& p, const StepArrays& a, void* stream, Laun
 // The classify kernel and the bucket scan (work records, length buckets and their offsets,
 // general-path worklist, bulk copies): the adjoint reverses the lists they leave.  Returns the number of classify blocks (the slices of
 // the buckets) or a negative error.
-template <class R, int KS, int NS>
+template <class R, int NS>
 int launch_classify_ns(const StepParams& p, const StepArrays& a, void* stream)
 {
-    using Smem = TileSmem<R, KS, kTileTY>;
+    using Smem = TileSmem<R, kTileTY>;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     int xchunk = 0, gz = 0, gy = 0, gx = 0;
     tiled_geometry(p.nx, p.ny, p.nz, &xchunk, &gz, &gy, &gx);
-    auto kern = tile_classify_kernel<R, KS, kTileTY, NS>;
+    auto kern = tile_classify_kernel<R, kTileTY, NS>;
     const size_t smem = sizeof(Smem);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return -(int)e;
@@ -1004,16 +1050,9 @@ int launch_classify_ns(const StepParams& p, const StepArrays& a, void* stream)
 }
 
 template <class R>
-int launch_classify(const StepParams& p, const StepArrays& a, int k_slots, void* stream)
+int launch_classify(const StepParams& p, const StepArrays& a, void* stream)
 {
-    const bool ns27 = p.ns == 27;
-    switch (k_slots)
-    {
-        case 8:  return ns27 ? launch_classify_ns<R, 8, 27>(p, a, stream) : launch_classify_ns<R, 8, 7>(p, a, stream);
-        case 12: return ns27 ? launch_classify_ns<R, 12, 27>(p, a, stream) : launch_classify_ns<R, 12, 7>(p, a, stream);
-        case 16: return ns27 ? launch_classify_ns<R, 16, 27>(p, a, stream) : launch_classify_ns<R, 16, 7>(p, a, stream);
-        default: return -1;
-    }
+    return p.ns == 27 ? launch_classify_ns<R, 27>(p, a, stream) : launch_classify_ns<R, 7>(p, a, stream);
 }
 
 template <class R, int KS, int KL>
