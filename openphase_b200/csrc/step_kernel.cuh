@@ -66,17 +66,28 @@ __device__ __forceinline__ double limited_force(const StepParams& p, const StepA
     return locdG;
 }
 
+// The limited force of a pair that averaging leaves none: the limiter of zero, which is zero (NaN for
+// an allowed force of zero, as 0 * tanh(0 / 0) of the reference's limiter).
+__device__ __forceinline__ double no_force(const StepParams& p, const StepArrays& a, int ga, int gb)
+{
+    if (p.limiting && p.allowed_p[a.gphase[ga] * p.nphases + a.gphase[gb]] == 0.0) return nan("");
+    return 0.0;
+}
+
+// Bit of the pair (i, j), i < j, of stored fields in a voxel's averaging mask.
+__device__ __forceinline__ constexpr int avg_bit(int i, int j) { return j * (j - 1) / 2 + i; }
+
 // The limited driving force of list entries i < j of an interface voxel v with c stored fields (the
-// leading entries of its list): with driving-force averaging, the averaged force of a pair of
-// stored fields; else, and for the zero-valued candidates (weight 0: their force is multiplied by
-// 0 unless a Seed takes part, which the reference gives the raw force), the pair's own force.
+// leading entries of its list): the pair's own force; with driving-force averaging a pair of stored
+// fields has it only where its bit is set.  (The zero-valued candidates have weight 0: their force
+// is multiplied by 0 unless a Seed takes part, which the reference gives the raw force.)
 __device__ __forceinline__ double pair_force(const StepParams& p, const StepArrays& a, long long v, int c, int i,
                                              int j, int gi, int gj)
 {
-    if (a.df_lim && j < c)
+    if (a.avg_mask && j < c)
     {
-        const unsigned o = a.df_off[v];
-        if ((unsigned long long)o + (unsigned)(c * (c - 1) / 2) <= a.df_cap) return a.df_lim[o + pair_pos(i, j, c)];
+        const int bit = avg_bit(i, j);
+        if (!((a.avg_mask[(long long)(bit >> 5) * p.n + v] >> (bit & 31)) & 1u)) return no_force(p, a, gi, gj);
     }
     return limited_force(p, a, gi, gj);
 }

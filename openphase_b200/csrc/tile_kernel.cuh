@@ -620,8 +620,9 @@ constexpr int kVolCache = 4;       // per-thread grain-volume cache of the compu
 // range (bucket_off); each CUDA block takes an equal contiguous part of it, its warps 32
 // consecutive entries at a time, so that no warp idles while another drains a long slice.
 //
-// N <= kListCap <= the stored fields per voxel, so a new record always fits.
-template <class R, int N>
+// N <= kListCap <= the stored fields per voxel, so a new record always fits.  AVG: averaged driving
+// forces (a template parameter: the mask costs the plain step registers).
+template <class R, int N, bool AVG>
 __global__ void __launch_bounds__(128) list_compute_kernel(const __grid_constant__ StepParams p, const StepArrays a,
                                                            int nslices)
 {
@@ -740,12 +741,20 @@ __global__ void __launch_bounds__(128) list_compute_kernel(const __grid_constant
         // ---- driving force (interface voxels only) ----------------------------------------------
         if (p.use_dg && flag == 2)
         {
+            // stored fields are positive: the pairs of two of them are the ones averaging decides on
+            unsigned reached = 0;
+            if constexpr (AVG) reached = a.avg_mask[v];
 #pragma unroll
             for (int i = 0; i < N; i++)
 #pragma unroll
                 for (int j = i + 1; j < N; j++)
                 {
-                    const double locdG = limited_force(p, a, g[i], g[j]);
+                    double locdG;
+                    if constexpr (AVG)
+                        locdG = val[j] != R(0) && !((reached >> avg_bit(i, j)) & 1u) ? no_force(p, a, g[i], g[j])
+                                                                                    : limited_force(p, a, g[i], g[j]);
+                    else
+                        locdG = limited_force(p, a, g[i], g[j]);
                     double norm = sqrt((double)val[i] * (double)val[j]);
                     if (a.gstage[g[i]] == 1 || a.gstage[g[j]] == 1) norm += 1.0e-6;
                     const double dpsi = locdG * (double)(R)pair_mobility(p, a, g[i], g[j]) * norm * p.pref_df;
@@ -980,17 +989,17 @@ struct SideFork {
 // stream -> side streams (FP64, us): 64^3 337 -> 192, 128^3 1024 -> 794, 192^3 2520 -> 2355, 224^3
 // 3749 -> 3690, 256^3 5465 -> 5600: the line lies between the last two.
 constexpr long long kSideVoxels = 12000000;
-template <class R>
+template <class R, bool AVG>
 void launch_lists(const StepParams& p, const StepArrays& a, int cb, int nblocks, const SideFork& fork)
 {
     const cudaStream_t s = fork.main;
-    list_compute_kernel<R, 8><<<cb, 128, 0, fork.on(0)>>>(p, a, nblocks);
-    list_compute_kernel<R, 7><<<cb, 128, 0, fork.on(1)>>>(p, a, nblocks);
-    list_compute_kernel<R, 6><<<cb, 128, 0, s>>>(p, a, nblocks);
-    list_compute_kernel<R, 5><<<cb, 128, 0, fork.on(3)>>>(p, a, nblocks);
-    list_compute_kernel<R, 4><<<cb, 128, 0, s>>>(p, a, nblocks);
-    list_compute_kernel<R, 3><<<cb, 128, 0, fork.on(3)>>>(p, a, nblocks);
-    list_compute_kernel<R, 2><<<cb, 128, 0, fork.on(1)>>>(p, a, nblocks);
+    list_compute_kernel<R, 8, AVG><<<cb, 128, 0, fork.on(0)>>>(p, a, nblocks);
+    list_compute_kernel<R, 7, AVG><<<cb, 128, 0, fork.on(1)>>>(p, a, nblocks);
+    list_compute_kernel<R, 6, AVG><<<cb, 128, 0, s>>>(p, a, nblocks);
+    list_compute_kernel<R, 5, AVG><<<cb, 128, 0, fork.on(3)>>>(p, a, nblocks);
+    list_compute_kernel<R, 4, AVG><<<cb, 128, 0, s>>>(p, a, nblocks);
+    list_compute_kernel<R, 3, AVG><<<cb, 128, 0, fork.on(3)>>>(p, a, nblocks);
+    list_compute_kernel<R, 2, AVG><<<cb, 128, 0, fork.on(1)>>>(p, a, nblocks);
 }
 
 template <class R, int KS, int KL, int NS>
@@ -1021,7 +1030,8 @@ int launch_tiled_ns(const StepParams& p, const StepArrays& a, void* stream, Laun
     if (e != cudaSuccess) return (int)e;
     const SideFork fork(info && p.n <= kSideVoxels ? info->side : nullptr, s);
     gk<<<148 * 4, 128, wsm, fork.on(2)>>>(p, a);
-    launch_lists<R>(p, a, cb, nblocks, fork);
+    if (a.avg_mask) launch_lists<R, true>(p, a, cb, nblocks, fork);
+    else launch_lists<R, false>(p, a, cb, nblocks, fork);
     if ((e = fork.join()) != cudaSuccess) return (int)e;
     if (info) info->kernels += 10;
     return (int)cudaGetLastError();
@@ -1067,11 +1077,10 @@ template <class R>
 int launch_step(const StepParams& p, const StepArrays& a, int k_slots, int variant, void* stream,
                 LaunchInfo* info)
 {
-    if (variant == kVariantGeneric || p.aniso || a.df_lim)
+    if (variant == kVariantGeneric || p.aniso)
     {
-        // anisotropic energies need the gradients of every list entry, and the averaged driving
-        // force is read per voxel pair: the per-voxel generic kernel only (the tiled kernels stay
-        // free of both)
+        // anisotropic energies need the gradients of every list entry: the per-voxel generic kernel
+        // only (the tiled kernels stay free of them)
         if (info) info->kernels += 1;
         return launch_step_generic<R>(p, a, k_slots, stream);
     }

@@ -73,3 +73,49 @@ def test_averaging_refused_where_unsupported():
     with pytest.raises(OpgpuError) as e:
         R.backward(np.ones(case.ngrains))
     assert e.value.code & E_INVALID
+
+
+# junction-dense small grains (up to 13 fields a voxel: every word of the pair mask; VolumeRatio < 1
+# lowers the threshold, so voxels hold several pairs above it), and boxes the sphere wraps around
+DENSE = {
+    "dense": Case(24, 24, 24, 30, seed=7, iwidth=6.0, dt=0.08, sigma=1.2, sigma_pairs=(0.8, 0.4), dg_scale=0.05,
+                  average=True, name="dense"),
+    "thin_box": Case(26, 11, 5, 6, seed=13, iwidth=6.0, dt=0.08, dg_scale=0.1, average=True, name="thin_box"),
+    "narrow": Case(24, 20, 22, 9, seed=17, iwidth=4.0, dt=0.08, dg_scale=0.1, average=True, name="narrow"),
+}
+
+
+@pytest.mark.parametrize("name", list(DENSE))
+@pytest.mark.parametrize("variant", ["tiled", "generic"])
+def test_averaging_dense_and_wrapped_grids(name, variant):
+    case = DENSE[name]
+    state = case.initial_state()
+    ctx = Context.from_case(case, precision="fp64", k_slots=16, state=state)
+    ctx.set_kernel_variant(variant)
+    ora = Oracle(case, *state)
+    for _ in range(4):
+        ctx.step(case.dt, 1)
+        ora.step(1)
+        r = compare_states(ctx.download(), ora.state(positive_only=True), case.ngrains)
+        assert r["non_borderline_mismatch_voxels"] == 0 and r["max_dphi"] <= TOL, r
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("threshold", [0.0, 0.02])
+def test_averaging_tiled_equals_generic(precision, threshold):
+    """Both kernels read the same mask: large grains (VolumeRatio = 1) give identical lists in either
+    precision, the FP64 values bit for bit; a low threshold makes most marks "several"."""
+    case = Case(40, 33, 37, 10, seed=19, iwidth=5.0, dt=0.08, dg_scale=0.1, average=True, name="tiled_generic")
+    state = case.initial_state()
+    got = []
+    for variant in ("tiled", "generic"):
+        ctx = Context.from_case(case, precision=precision, k_slots=12, state=state)
+        ctx.set_averaging(True, 0, threshold)
+        ctx.set_kernel_variant(variant)
+        ctx.step(case.dt, 3)
+        got.append(ctx.download())
+    r = compare_states(*got, case.ngrains)
+    if precision == "fp64":
+        assert r["same_sets"] and r["max_dphi"] == 0.0, r
+    else:
+        assert r["max_dphi"] <= 1e-3, r   # FP32 Laplacians are fused in one and not in the other
