@@ -1001,12 +1001,11 @@ adjoint_gather_kernel(const __grid_constant__ StepParams p, const StepArrays la,
 
     for (int i = t; i < kSlots * 3 * Geo::kRecs; i += NT) (&S.dense[0][0][0])[i] = 0.0;
     for (int i = t; i < 3 * Geo::kRecs; i += NT) (&S.word[0][0])[i] = 0u;
-    if (t < kSlots) { S.grain_of[t] = -1; S.lastpos[t] = -1000; }
-    if (t < kSlotHash) S.hkey[t] = -1;
+    if (t < 16) { S.grain_of[t] = -1; S.lastpos[t] = -1000; }
+    for (int i = t; i < kSlotMap; i += NT) S.map[i] = 0;
     if (t < 32) S.pending[t] = -1;
-    if (t == 0) S.tomb = 0;
-    int cr[PlaneRegs<TY>::kPer];
-    prefetch_counts<TY>(p, la, x0 == 0 ? nx - 1 : x0 - 1, y0, z0, t, cr);
+    PlaneState<TY> P;
+    plane_begin<TY>(p, la, x0 == 0 ? nx - 1 : x0 - 1, y0, z0, t, P);
     __syncthreads();
 
     const int rec0 = (ty + 1) * kC + (tz + 1);
@@ -1016,7 +1015,7 @@ adjoint_gather_kernel(const __grid_constant__ StepParams p, const StepArrays la,
         int xp = x0 - 1 + j;
         xp = xp < 0 ? xp + nx : (xp >= nx ? xp - nx : xp);
         if (j > 0) __syncthreads();
-        load_plane(p, la, S, j % 3, xp, j - 1, y0, z0, t, cr);
+        load_plane(p, la, S, j % 3, xp, j - 1, t, P);
         __syncthreads();
         if (j < 2 || !inside) continue;
         const int x = x0 + j - 2;
@@ -1044,7 +1043,7 @@ adjoint_gather_kernel(const __grid_constant__ StepParams p, const StepArrays la,
             }
             else
             {
-                const int k = find_slot(S.hkey, S.hslot, g);
+                const int k = find_slot(S, g);
                 if (k >= 0)
                 {
 #pragma unroll

@@ -35,19 +35,13 @@ template <class R>
 struct WindowSlots {
     static constexpr int value = sizeof(R) == 8 ? 14 : 16;
 };
-constexpr int kSlotHash = 64;        // grain -> slot hash table entries
+constexpr int kSlotMap = 512;        // grain -> slot map entries
 constexpr int kTileVolSlots = 512;      // grain-volume hash of the compute kernels
 constexpr int kKeepEntries = 6;         // entries per record the plane loader keeps in registers
-// The FP64 plane loader keeps the slots step 1 found in shared memory for step 3 (measured 5 %
-// faster classify); in FP32 the extra addressing costs more than the second hash lookup saves.
-template <class R>
-struct LoaderSlotCache {
-    static constexpr bool value = sizeof(R) == 8;
-};
-// grain-volume hash of the classify kernel (bulk voxels); smaller where the slot cache needs room
+// grain-volume hash of the classify kernel (bulk voxels); smaller where the dense planes need room
 template <class R>
 struct ClassifyVolSlots {
-    static constexpr int value = LoaderSlotCache<R>::value ? 128 : 256;
+    static constexpr int value = sizeof(R) == 8 ? 128 : 256;
 };
 // Blocks of each per-length compute kernel: one per 4096 voxels of the grid, between 8 and 32 per
 // SM (a finer split of each length's entries pays on large grids; on small ones the per-block
@@ -67,32 +61,31 @@ struct TileGeom {
     static constexpr int NT = kTileZ * TY;
 };
 
+// Flags of a record's word beside its slot bitmask.
+constexpr uint32_t kWordSeveral = 0x80000000u;     // more than one field
+constexpr uint32_t kWordUnslotted = 0x40000000u;   // a grain of the record has no slot
+
 template <class R, int TY>
 struct TileSmem {
     using Geo = TileGeom<TY>;
     static constexpr int kSlots = WindowSlots<R>::value;
     R dense[kSlots][3][Geo::kRecs];          // per-slot values of the three ring planes (zero where absent)
     double vol_sum[ClassifyVolSlots<R>::value];
-    uint64_t slotl[3][Geo::kRecs];           // slot ids of the record in entry order, 4 bits each
-    uint32_t word[3][Geo::kRecs];            // slot bitmask of the record | (more than one field) << 31
-                                             // | (a grain of the record has no slot) << 30
+    uint2 slotl[3][Geo::kRecs];              // slot ids of the record in entry order, 4 bits each
+    uint32_t word[3][Geo::kRecs];            // slot bitmask of the record | kWordSeveral | kWordUnslotted
     int vol_key[ClassifyVolSlots<R>::value];
-    int grain_of[kSlots];                    // slot -> grain (-1 = free)
-    int lastpos[kSlots];                     // last window position where the slot's grain occurs
-    int hkey[kSlotHash];                     // grain -> slot hash: key (-1 empty, -2 deleted)
+    alignas(16) int grain_of[16];            // slot -> grain (-1 = free or beyond kSlots)
+    int lastpos[16];                         // last window position where the slot's grain occurs
     int pending[32];                         // grains of the incoming plane that need a slot
     unsigned nb[kListCap + 1];               // entries this block appended per list length
     unsigned woff;                           // bytes of work records this block wrote
     unsigned crowded;                        // voxels sent to the general path for a crowded window
     unsigned long long cnt[3];
-    uint8_t hslot[kSlotHash];                // grain -> slot hash: slot
+    uint8_t map[kSlotMap];                   // hashed grain -> a slot that may hold it (check grain_of)
     uint8_t cntr[3][Geo::kRecs];             // entries per record
-    uint8_t pslot[LoaderSlotCache<R>::value ? Geo::kRecs : 1][kKeepEntries];   // slot step 1 found per kept
-                                                                             // entry (0xFF: none)
-    uint8_t tomb;                            // deleted hash entries
 };
 
-__device__ __forceinline__ unsigned slot_hash(int g) { return ((unsigned)g * 2654435761u) >> 26; }
+__device__ __forceinline__ unsigned slot_hash(int g) { return ((unsigned)g * 2654435761u) >> 23; }
 
 // One term of the classify kernel's dense-plane Laplacian.  FP64: the reference's separate multiply
 // and add (the FP64 unit is compiled without contraction).  FP32: one fused multiply-add, written
@@ -102,39 +95,30 @@ __device__ __forceinline__ unsigned slot_hash(int g) { return ((unsigned)g * 265
 __device__ __forceinline__ double lap_acc(double l, double w, double x) { return l + w * x; }
 __device__ __forceinline__ float lap_acc(float l, float w, float x) { return __fmaf_rn(w, x, l); }
 
-// Slot of a grain in the window (-1 if the grain has none).
-__device__ __forceinline__ int find_slot(const int* hkey, const uint8_t* hslot, int g)
+// Slot of a grain in the window (-1 if the grain has none).  A window holds at most 16 grains, so
+// the map hits but for a few per cent of the grains, whose entry another grain of the window took;
+// they are searched for among the slots.
+template <class S>
+__device__ __forceinline__ int search_slot(const S& sm, int g)
 {
-    unsigned h = slot_hash(g);
-    for (int probe = 0; probe < kSlotHash; probe++)
+    int k = -1;
+#pragma unroll
+    for (int q = 0; q < 4; q++)
     {
-        const int k = hkey[h];
-        if (k == g) return hslot[h];
-        if (k == -1) return -1;
-        h = (h + 1) & (kSlotHash - 1);
+        const int4 four = reinterpret_cast<const int4*>(sm.grain_of)[q];
+        if (four.x == g) k = 4 * q;
+        if (four.y == g) k = 4 * q + 1;
+        if (four.z == g) k = 4 * q + 2;
+        if (four.w == g) k = 4 * q + 3;
     }
-    return -1;
+    return k;
 }
 
-__device__ __forceinline__ void hash_insert(int* hkey, uint8_t* hslot, int g, int slot)
+template <class S>
+__device__ __forceinline__ int find_slot(const S& sm, int g)
 {
-    unsigned h = slot_hash(g);
-    for (int probe = 0; probe < kSlotHash; probe++)
-    {
-        if (hkey[h] < 0) { hkey[h] = g; hslot[h] = (uint8_t)slot; return; }
-        h = (h + 1) & (kSlotHash - 1);
-    }
-}
-
-__device__ __forceinline__ void hash_erase(int* hkey, int g, uint8_t& tomb)
-{
-    unsigned h = slot_hash(g);
-    for (int probe = 0; probe < kSlotHash; probe++)
-    {
-        if (hkey[h] == g) { hkey[h] = -2; tomb++; return; }
-        if (hkey[h] == -1) return;
-        h = (h + 1) & (kSlotHash - 1);
-    }
+    const int k = sm.map[slot_hash(g)];
+    return sm.grain_of[k] == g ? k : search_slot(sm, g);
 }
 
 // Records of a ring plane each thread handles, and how many entries of each it keeps in registers
@@ -145,109 +129,145 @@ struct PlaneRegs {
     static constexpr int kKeep = kKeepEntries;
 };
 
+// In-plane offset of record r (the same in every plane; -1 beyond the last record).
 template <int TY>
-__device__ __forceinline__ long long plane_voxel(const StepParams& p, long long base, int r, int y0, int z0)
+__device__ __forceinline__ int record_offset(const StepParams& p, int r, int y0, int z0)
 {
     using Geo = TileGeom<TY>;
+    if (r >= Geo::kRecs) return -1;
     const int row = r / Geo::kCols, col = r - row * Geo::kCols;
     int yy = y0 - 1 + row; yy = yy < 0 ? yy + p.ny : (yy >= p.ny ? yy % p.ny : yy);
     int zz = z0 - 1 + col; zz = zz < 0 ? zz + p.nz : (zz >= p.nz ? zz % p.nz : zz);
-    return base + (long long)yy * p.nz + zz;
+    return yy * p.nz + zz;
 }
+
+// What a thread of the plane loader keeps from plane to plane: the in-plane offsets of its records
+// and the next plane's counts (prefetched).
+template <int TY>
+struct PlaneState {
+    int off[PlaneRegs<TY>::kPer];
+    int cr[PlaneRegs<TY>::kPer];
+};
 
 // Counts of plane xp for this thread's records (issued one plane ahead of their use).
 template <int TY>
-__device__ __forceinline__ void prefetch_counts(const StepParams& p, const StepArrays& a, int xp, int y0, int z0,
-                                                int t, int (&cr)[PlaneRegs<TY>::kPer])
+__device__ __forceinline__ void prefetch_counts(const StepParams& p, const StepArrays& a, int xp, PlaneState<TY>& P)
 {
-    using Geo = TileGeom<TY>;
-    const long long base = (long long)xp * p.ny * p.nz;
+    const uint8_t* __restrict__ cnt = a.cnt_in + (long long)xp * p.ny * p.nz;
 #pragma unroll
-    for (int i = 0; i < PlaneRegs<TY>::kPer; i++)
-    {
-        const int r = t + i * Geo::NT;
-        cr[i] = r < Geo::kRecs ? (int)a.cnt_in[plane_voxel<TY>(p, base, r, y0, z0)] : 0;
-    }
+    for (int i = 0; i < PlaneRegs<TY>::kPer; i++) P.cr[i] = P.off[i] >= 0 ? (int)cnt[P.off[i]] : 0;
 }
 
-// Registers a thread keeps between the passes of the plane loader: the voxel index of each of its
-// records and their first kKeep entries.
+// The loader state of a thread before its first plane xp.
+template <int TY>
+__device__ __forceinline__ void plane_begin(const StepParams& p, const StepArrays& a, int xp, int y0, int z0, int t,
+                                            PlaneState<TY>& P)
+{
+#pragma unroll
+    for (int i = 0; i < PlaneRegs<TY>::kPer; i++) P.off[i] = record_offset<TY>(p, t + i * TileGeom<TY>::NT, y0, z0);
+    prefetch_counts<TY>(p, a, xp, P);
+}
+
+// Registers a thread keeps between the passes of the plane loader: the first kKeep entries of each
+// of its records, the slots found so far (4 bits an entry, entries 0-7 and 8-15) and the entries
+// without one.
 template <class R, int TY>
 struct PlaneLoad {
-    long long vv[PlaneRegs<TY>::kPer];
     int gr[PlaneRegs<TY>::kPer][PlaneRegs<TY>::kKeep];
     R vr[PlaneRegs<TY>::kPer][PlaneRegs<TY>::kKeep];
+    uint32_t lst[PlaneRegs<TY>::kPer][2];
+    uint32_t miss[PlaneRegs<TY>::kPer];
 };
+
+// Grain of entry s of record i (the kept ones without a dynamic register index).
+template <class R, int TY>
+__device__ __forceinline__ int kept_grain(const PlaneLoad<R, TY>& L, int i, int s, const int16_t* __restrict__ gin,
+                                          long long N)
+{
+    int g = 0;
+#pragma unroll
+    for (int q = 0; q < PlaneRegs<TY>::kKeep; q++)
+        if (q == s) g = L.gr[i][q];
+    return s >= PlaneRegs<TY>::kKeep ? (int)gin[s * N] : g;
+}
 
 // Bringing plane xp (window position wpos) into ring slot `rs` -- slot lists, bitmask words and
 // dense per-slot values; grains not yet in the window get a slot that no grain of the window uses --
 // takes three passes with a barrier between each:
-//   plane_scan    reads the records once (the first kKeep entries stay in registers), marks the
-//                 grains already slotted as in use and collects the others in `pending`; it touches
-//                 only the hash (read), lastpos, pslot and pending, so it may run while other
-//                 threads still read the ring for the previous plane; returns whether this thread
-//                 added a pending grain
+//   plane_scan    reads the records once (the first kKeep entries stay in registers) and finds their
+//                 slots through the map; marks the slots as in use and collects the grains without
+//                 one in `pending`; it touches only map and grain_of (read), lastpos and pending, so
+//                 it may run while other threads still read the ring for the previous plane; returns
+//                 whether this thread added a pending grain
 //   plane_assign  warp 0 hands free slots to the pending grains (only needed when some thread
 //                 added one)
 //   plane_fill    slot lists, bitmask words and dense values of the incoming plane, clearing what
-//                 the ring position held before
-// cr holds the plane's counts on entry (prefetched) and the next plane's counts after plane_fill.
+//                 the ring position held before and no longer holds
+// P.cr holds the plane's counts on entry (prefetched) and the next plane's counts after plane_fill.
 // Invariant of the dense planes: dense[k][rs][r] != 0 only if bit k of word[rs][r] is set.
 template <class R, int TY>
 __device__ __forceinline__ bool plane_scan(const StepParams& p, const StepArrays& a, TileSmem<R, TY>& S,
-                                           int xp, int wpos, int y0, int z0, int t,
-                                           const int (&cr)[PlaneRegs<TY>::kPer], PlaneLoad<R, TY>& L)
+                                           int xp, int wpos, const PlaneState<TY>& P, PlaneLoad<R, TY>& L)
 {
-    using Geo = TileGeom<TY>;
     using PR = PlaneRegs<TY>;
     const long long N = p.n;
     const long long base = (long long)xp * p.ny * p.nz;
-    const R* __restrict__ vin = static_cast<const R*>(a.val_in);
+    const int16_t* __restrict__ gin = a.idx_in + base;
+    const R* __restrict__ vin = static_cast<const R*>(a.val_in) + base;
     bool added = false;
 #pragma unroll
     for (int i = 0; i < PR::kPer; i++)
-    {
-        const int r = t + i * Geo::NT;
-        L.vv[i] = r < Geo::kRecs ? plane_voxel<TY>(p, base, r, y0, z0) : 0;
 #pragma unroll
         for (int s = 0; s < PR::kKeep; s++)
-        {
-            if (s < cr[i])
+            if (s < P.cr[i])
             {
-                L.gr[i][s] = a.idx_in[s * N + L.vv[i]];
-                L.vr[i][s] = vin[s * N + L.vv[i]];
+                L.gr[i][s] = gin[s * N + P.off[i]];
+                L.vr[i][s] = vin[s * N + P.off[i]];
             }
-        }
-    }
 #pragma unroll
     for (int i = 0; i < PR::kPer; i++)
     {
-        for (int s = 0; s < cr[i]; s++)
-        {
-            int g;
+        const int c = P.cr[i];
+        uint32_t lst[2] = {0u, 0u};
+        uint32_t miss = c > PR::kKeep ? ((1u << c) - 1u) & ~((1u << PR::kKeep) - 1u) : 0u;
 #pragma unroll
-            for (int q = 0; q < PR::kKeep; q++)
-                if (q == s) g = L.gr[i][q];
-            if (s >= PR::kKeep) g = a.idx_in[s * N + L.vv[i]];
-            const int k0 = find_slot(S.hkey, S.hslot, g);
-            if constexpr (LoaderSlotCache<R>::value)
-                if (s < PR::kKeep) S.pslot[t + i * Geo::NT][s] = (uint8_t)(k0 >= 0 ? k0 : 0xFF);
-            if (k0 >= 0)
+        for (int s = 0; s < PR::kKeep; s++)
+            if (s < c)
             {
-                S.lastpos[k0] = wpos;   // in use by the incoming plane: not free for plane_assign
-            }
-            else
-            {
-                added = true;
-                unsigned h = ((unsigned)g * 2654435761u) & 31u;
-                for (int probe = 0; probe < 32; probe++)
+                const int g = L.gr[i][s], k = S.map[slot_hash(g)];
+                if (S.grain_of[k] == g)
                 {
-                    const int k = atomicCAS(&S.pending[h], -1, g);
-                    if (k == -1 || k == g) break;
-                    h = (h + 1) & 31u;
+                    S.lastpos[k] = wpos;   // in use by the incoming plane: not free for plane_assign
+                    lst[0] |= (uint32_t)k << (4 * s);
                 }
+                else miss |= 1u << s;
+            }
+        uint32_t left = 0;
+        for (uint32_t m = miss; m; m &= m - 1u)
+        {
+            const int s = __ffs(m) - 1;
+            const int g = kept_grain<R, TY>(L, i, s, gin + P.off[i], N);
+            const int k = search_slot(S, g);
+            if (k >= 0)
+            {
+                S.lastpos[k] = wpos;
+                if (s < 8) lst[0] |= (uint32_t)k << (4 * s);
+                else lst[1] |= (uint32_t)k << (4 * s - 32);
+                continue;
+            }
+            added = true;
+            left |= 1u << s;
+            unsigned h = ((unsigned)g * 2654435761u) & 31u;
+            for (int probe = 0; probe < 32; probe++)
+            {
+                const int q = atomicCAS(&S.pending[h], -1, g);
+                if (q == -1 || q == g) break;
+                h = (h + 1) & 31u;
             }
         }
+        L.lst[i][0] = lst[0];
+        L.lst[i][1] = lst[1];
+        L.miss[i] = left;
     }
     return added;
 }
@@ -255,101 +275,93 @@ __device__ __forceinline__ bool plane_scan(const StepParams& p, const StepArrays
 template <class R, int TY>
 __device__ __forceinline__ void plane_assign(TileSmem<R, TY>& S, int wpos, int t)
 {
-    // warp 0 hands free slots (grain gone from the window) to the pending grains; lane 0 keeps
-    // the grain -> slot hash in step
+    // warp 0 hands free slots (grain gone from the window) to the pending grains
     if (t < 32)
     {
         const int g = S.pending[t];
         const bool valid = g >= 0;
         constexpr int kSlots = WindowSlots<R>::value;
-        const bool is_free = t < kSlots && (S.grain_of[t] < 0 || S.lastpos[t] < wpos - 2);
+        const bool is_free = t < kSlots && (S.grain_of[t & 15] < 0 || S.lastpos[t & 15] < wpos - 2);
         const unsigned fm = __ballot_sync(0xffffffffu, is_free);
         const unsigned vm = __ballot_sync(0xffffffffu, valid);
         const int rank = __popc(vm & ((1u << t) - 1u));
-        const int k = (valid && rank < __popc(fm)) ? (int)__fns(fm, 0, rank + 1) : -1;
-        if (valid) S.pending[t] = -1;
-        for (unsigned m = vm; m; m &= m - 1u)
-        {
-            const int lane = __ffs(m) - 1;
-            const int gl = __shfl_sync(0xffffffffu, g, lane);
-            const int kl = __shfl_sync(0xffffffffu, k, lane);
-            if (t == 0 && kl >= 0)
-            {
-                const int old = S.grain_of[kl];
-                if (old >= 0) hash_erase(S.hkey, old, S.tomb);
-                hash_insert(S.hkey, S.hslot, gl, kl);
-                S.grain_of[kl] = gl;
-                S.lastpos[kl] = wpos;
-            }
-        }
         // grains left without a slot are marked per record in plane_fill
-        if (t == 0 && S.tomb > 24)
+        if (valid)
         {
-            for (int h = 0; h < kSlotHash; h++) S.hkey[h] = -1;
-            for (int q = 0; q < kSlots; q++)
-                if (S.grain_of[q] >= 0) hash_insert(S.hkey, S.hslot, S.grain_of[q], q);
-            S.tomb = 0;
+            S.pending[t] = -1;
+            if (rank < __popc(fm))
+            {
+                const int k = (int)__fns(fm, 0, rank + 1);
+                S.grain_of[k] = g;
+                S.lastpos[k] = wpos;
+                S.map[slot_hash(g)] = (uint8_t)k;
+            }
         }
     }
 }
 
 template <class R, int TY>
 __device__ __forceinline__ void plane_fill(const StepParams& p, const StepArrays& a, TileSmem<R, TY>& S,
-                                           int rs, int xp, int y0, int z0, int t, int (&cr)[PlaneRegs<TY>::kPer],
-                                           const PlaneLoad<R, TY>& L)
+                                           int rs, int xp, int t, PlaneState<TY>& P, const PlaneLoad<R, TY>& L)
 {
     using Geo = TileGeom<TY>;
     using PR = PlaneRegs<TY>;
     const long long N = p.n;
-    const R* __restrict__ vin = static_cast<const R*>(a.val_in);
+    const long long base = (long long)xp * p.ny * p.nz;
+    const R* __restrict__ vin = static_cast<const R*>(a.val_in) + base;
 #pragma unroll
     for (int i = 0; i < PR::kPer; i++)
     {
         const int r = t + i * Geo::NT;
         if (r >= Geo::kRecs) continue;
-        for (uint32_t m = S.word[rs][r] & 0xFFFFu; m; m &= m - 1u) S.dense[__ffs(m) - 1][rs][r] = R(0);
-        uint32_t msk = 0;
-        uint64_t lst = 0;
-        bool unslotted = false;
-        const int c = cr[i];
-        for (int s = 0; s < c; s++)
+        const int c = P.cr[i];
+        uint32_t lst[2] = {L.lst[i][0], L.lst[i][1]};
+        // the slots plane_assign handed out
+        uint32_t lost = 0;
+        for (uint32_t m = L.miss[i]; m; m &= m - 1u)
         {
-            int g;
-            R val;
-#pragma unroll
-            for (int q = 0; q < PR::kKeep; q++)
-                if (q == s) { g = L.gr[i][q]; val = L.vr[i][q]; }
-            if (s >= PR::kKeep) { g = a.idx_in[s * N + L.vv[i]]; val = vin[s * N + L.vv[i]]; }
-            // the slot plane_scan found, else the one plane_assign handed out
-            int k = 0xFF;
-            if constexpr (LoaderSlotCache<R>::value)
-                if (s < PR::kKeep) k = S.pslot[r][s];
-            if (k == 0xFF) k = find_slot(S.hkey, S.hslot, g);
-            if (k < 0) { unslotted = true; continue; }
-            S.dense[k][rs][r] = val;
-            lst |= (uint64_t)k << (4 * s);
-            msk |= 1u << k;
+            const int s = __ffs(m) - 1;
+            const int k = search_slot(S, kept_grain<R, TY>(L, i, s, a.idx_in + base + P.off[i], N));
+            if (k < 0) lost |= 1u << s;
+            else if (s < 8) lst[0] |= (uint32_t)k << (4 * s);
+            else lst[1] |= (uint32_t)k << (4 * s - 32);
         }
-        S.word[rs][r] = msk | (c > 1 ? 0x80000000u : 0u) | (unslotted ? 0x40000000u : 0u);
-        S.slotl[rs][r] = lst;
+        uint32_t msk = 0;
+#pragma unroll
+        for (int s = 0; s < PR::kKeep; s++)
+            if (s < c && !((lost >> s) & 1u))
+            {
+                const int k = (int)(lst[0] >> (4 * s)) & 15;
+                S.dense[k][rs][r] = L.vr[i][s];
+                msk |= 1u << k;
+            }
+        for (int s = PR::kKeep; s < c; s++)
+            if (!((lost >> s) & 1u))
+            {
+                const int k = (int)(lst[s >> 3] >> (4 * (s & 7))) & 15;
+                S.dense[k][rs][r] = vin[s * N + P.off[i]];
+                msk |= 1u << k;
+            }
+        for (uint32_t m = S.word[rs][r] & 0xFFFFu & ~msk; m; m &= m - 1u) S.dense[__ffs(m) - 1][rs][r] = R(0);
+        S.word[rs][r] = msk | (c > 1 ? kWordSeveral : 0u) | (lost ? kWordUnslotted : 0u);
+        S.slotl[rs][r] = make_uint2(lst[0], lst[1]);
         S.cntr[rs][r] = (uint8_t)c;
     }
     // counts of the next plane, for the next call
-    prefetch_counts<TY>(p, a, xp == p.nx - 1 ? 0 : xp + 1, y0, z0, t, cr);
+    prefetch_counts<TY>(p, a, xp == p.nx - 1 ? 0 : xp + 1, P);
 }
 
 // The three passes with their barriers, for kernels that do not overlap plane_scan with other work.
 template <class R, int TY>
 __device__ __forceinline__ void load_plane(const StepParams& p, const StepArrays& a, TileSmem<R, TY>& S,
-                                           int rs, int xp, int wpos, int y0, int z0, int t,
-                                           int (&cr)[PlaneRegs<TY>::kPer])
+                                           int rs, int xp, int wpos, int t, PlaneState<TY>& P)
 {
     PlaneLoad<R, TY> L;
-    plane_scan(p, a, S, xp, wpos, y0, z0, t, cr, L);
+    plane_scan(p, a, S, xp, wpos, P, L);
     __syncthreads();
     plane_assign(S, wpos, t);
     __syncthreads();
-    plane_fill(p, a, S, rs, xp, y0, z0, t, cr, L);
+    plane_fill(p, a, S, rs, xp, t, P, L);
 }
 
 // Offsets of the q-th Laplacian stencil element (LaplacianStencil::Set order): 27-point stencils
@@ -361,26 +373,33 @@ __device__ __forceinline__ constexpr int stencil_dy(int q) { return NS == 27 ? (
 template <int NS>
 __device__ __forceinline__ constexpr int stencil_dz(int q) { return NS == 27 ? q % 3 - 1 : (q == 2 ? -1 : (q == 4 ? 1 : 0)); }
 
-// New grains of neighbour record (pl, r): append them (4-bit slot ids) in the record's entry order.
+// New grains of neighbour record (pl, r): append their slots (4 bits each) in the record's entry
+// order.  n counts on past kListCap, ls then holds no list.
 template <class R, int TY>
-__device__ __forceinline__ void append_fresh(const TileSmem<R, TY>& S, int pl, int r, uint32_t fresh,
-                                             uint64_t& ls, int& n, bool& over)
+__device__ __forceinline__ void append_fresh(const TileSmem<R, TY>& S, int pl, int r, uint32_t fresh, uint32_t& ls, int& n)
 {
-    const int cu = S.cntr[pl][r];
-    uint64_t lst = S.slotl[pl][r];
-    for (int s = 0; s < cu; s++, lst >>= 4)
+    if ((fresh & (fresh - 1u)) == 0u)
     {
-        const int k = (int)(lst & 15u);
+        // one new grain (the usual case): no order to look up
+        ls |= (uint32_t)(__ffs(fresh) - 1) << ((4 * n) & 31);
+        n++;
+        return;
+    }
+    const int cu = S.cntr[pl][r];
+    const uint2 list = S.slotl[pl][r];
+    for (int s = 0; s < cu; s++)
+    {
+        const uint32_t k = ((s < 8 ? list.x : list.y) >> (4 * (s & 7))) & 15u;
         if ((fresh >> k) & 1u)
         {
-            if (n < kListCap) { ls |= (uint64_t)k << (4 * n); n++; }
-            else over = true;
+            ls |= k << ((4 * n) & 31);
+            n++;
         }
     }
 }
 
 template <class R, int TY, int NS>
-__global__ void __launch_bounds__(kTileZ * TY)
+__global__ void __launch_bounds__(kTileZ * TY, sizeof(R) == 8 ? 3 : 5)
 tile_classify_kernel(const __grid_constant__ StepParams p, const StepArrays a, int xchunk)
 {
     using Geo = TileGeom<TY>;
@@ -408,21 +427,27 @@ tile_classify_kernel(const __grid_constant__ StepParams p, const StepArrays a, i
     constexpr int kSlots = WindowSlots<R>::value;
     for (int i = t; i < kSlots * 3 * Geo::kRecs; i += NT) (&S.dense[0][0][0])[i] = R(0);
     for (int i = t; i < 3 * Geo::kRecs; i += NT) (&S.word[0][0])[i] = 0u;
-    if (t < kSlots) { S.grain_of[t] = -1; S.lastpos[t] = -1000; }
-    if (t < kSlotHash) S.hkey[t] = -1;
+    if (t < 16) { S.grain_of[t] = -1; S.lastpos[t] = -1000; }
+    for (int i = t; i < kSlotMap; i += NT) S.map[i] = 0;
     if (t < 32) S.pending[t] = -1;
     if (t <= kListCap) S.nb[t] = 0u;
     if (t < 3) S.cnt[t] = 0ull;
-    if (t == 0) { S.woff = 0u; S.crowded = 0u; S.tomb = 0; }
+    if (t == 0) { S.woff = 0u; S.crowded = 0u; }
     unsigned wide = 0, ein = 0, eout = 0;
     uint32_t st = 0;
     int acc_g = -1;        // bulk-voxel volume accumulator of this thread
     double acc_v = 0.0;
-    int cr[PlaneRegs<TY>::kPer];
-    prefetch_counts<TY>(p, a, x0 == 0 ? nx - 1 : x0 - 1, y0, z0, t, cr);
+    PlaneState<TY> P;
+    plane_begin<TY>(p, a, x0 == 0 ? nx - 1 : x0 - 1, y0, z0, t, P);
     __syncthreads();
 
     const int rec0 = (ty + 1) * kC + (tz + 1);
+    // words of the thread's column of records, kept while the block marches along x: per plane the
+    // words of the three rows ORed over z (row0: the plane before the centre, row1: the centre plane,
+    // row2: the plane after) and the middle word
+    uint32_t row0[3], row1[3], row2[3], mid0 = 0, mid1 = 0, mid2 = 0;
+#pragma unroll
+    for (int dy = 0; dy < 3; dy++) row0[dy] = row1[dy] = row2[dy] = 0;
 
     // plane x0-1+j goes to ring slot j%3 at window position j-1; once three planes are in, the
     // centre plane x = x0+j-2 is processed (one call site of the plane loader keeps the code small)
@@ -435,15 +460,26 @@ tile_classify_kernel(const __grid_constant__ StepParams p, const StepArrays a, i
         // its barrier also ends that work, and the slot hand-out runs only when a grain is new
         {
             PlaneLoad<R, TY> L;
-            const bool added = plane_scan(p, a, S, xp, j - 1, y0, z0, t, cr, L);
+            const bool added = plane_scan(p, a, S, xp, j - 1, P, L);
             if (__syncthreads_or(added))
             {
                 plane_assign(S, j - 1, t);
                 __syncthreads();
             }
-            plane_fill(p, a, S, j % 3, xp, y0, z0, t, cr, L);
+            plane_fill(p, a, S, j % 3, xp, t, P, L);
         }
         __syncthreads();
+        mid0 = mid1; mid1 = mid2;
+#pragma unroll
+        for (int dy = 0; dy < 3; dy++)
+        {
+            row0[dy] = row1[dy];
+            row1[dy] = row2[dy];
+            const uint32_t* w = &S.word[j % 3][rec0 + (dy - 1) * kC];
+            const uint32_t m = w[0];
+            if (dy == 1) mid2 = m;
+            row2[dy] = w[-1] | m | w[1];
+        }
         if (j < 2 || !inside) continue;
         const int x = x0 + j - 2;
         const int sl0 = (j - 2) % 3, sl1 = (j - 1) % 3, sl2 = j % 3;
@@ -451,48 +487,18 @@ tile_classify_kernel(const __grid_constant__ StepParams p, const StepArrays a, i
 
         const int c = S.cntr[sl1][rec0];
         ein += c;
-        // ---- flag and (27-point stencils) candidate discovery over the neighbours ----------------
-        // One unrolled pass over the 27 bitmask words: the flag bits, and the stencil positions
-        // whose record holds a grain not seen at an earlier position (nor in the voxel itself).
-        const uint32_t own = S.word[sl1][rec0] & 0xFFFFu;
-        uint32_t multi = 0, qfresh = 0;
-        {
-            uint32_t seen = own;
+        // ---- flag and candidate discovery over the neighbours ------------------------------------
+        // Candidates come in the reference's order: new grains of each neighbour in stencil order and
+        // neighbour-list order.  The rows of three z-neighbours that hold a grain not seen in an
+        // earlier row (nor in the voxel itself) are marked from the row words in registers; only
+        // their records are visited (the others add nothing to the list).
+        const uint32_t own = mid1 & 0xFFFFu;
+        uint32_t multi = 0;
 #pragma unroll
-            for (int q = 0; q < 27; q++)
-            {
-                const int pl = q < 9 ? sl0 : (q < 18 ? sl1 : sl2);
-                const int r = rec0 + ((q / 3) % 3 - 1) * kC + (q % 3 - 1);
-                const uint32_t w = S.word[pl][r];
-                multi |= w;
-                if (w & 0xFFFFu & ~seen) qfresh |= 1u << q;
-                seen |= w;
-            }
-        }
+        for (int dy = 0; dy < 3; dy++) multi |= row0[dy] | row1[dy] | row2[dy];
         // a neighbour holding a grain the window has no slot for: the general path
-        const bool window_bad = (multi >> 30) & 1u;
-        uint64_t ls = 0;
-        int n = c;
-        bool over = window_bad || c > kListCap;
-        if (!over) ls = S.slotl[sl1][rec0];   // c <= kListCap entries, unused nibbles are zero
-        // candidates in the reference's order: new grains of each neighbour in stencil order and
-        // neighbour-list order.  Only the positions marked above bring new grains; the words of the
-        // others add nothing to `seen`, so visiting the marked ones in order gives the same list.
-        if (NS == 27 && !over && qfresh)
-        {
-            uint32_t seen = own;
-            for (uint32_t m = qfresh; m; m &= m - 1u)
-            {
-                const int q = __ffs(m) - 1;
-                const int pl = q < 9 ? sl0 : (q < 18 ? sl1 : sl2);
-                const int r = rec0 + ((q / 3) % 3 - 1) * kC + (q % 3 - 1);
-                const uint32_t w = S.word[pl][r] & 0xFFFFu;
-                append_fresh(S, pl, r, w & ~seen, ls, n, over);
-                if (over) break;
-                seen |= w;
-            }
-        }
-        const int flag = c > 1 ? 2 : ((multi >> 31) ? 1 : 0);
+        const bool window_bad = (multi & kWordUnslotted) != 0u;
+        const int flag = c > 1 ? 2 : ((multi & kWordSeveral) ? 1 : 0);
         if (flag == 0)
         {
             // bulk voxel: carried over unchanged
@@ -520,20 +526,58 @@ tile_classify_kernel(const __grid_constant__ StepParams p, const StepArrays a, i
             continue;
         }
         wide++;
-        if (NS != 27 && !over)
+        uint32_t ls = 0;
+        int n = c;
+        bool over = window_bad || c > kListCap;
+        if (!over)
         {
-            // 7-point Laplacian: its stencil order, then the gradient pass over the 26 neighbours
+            ls = S.slotl[sl1][rec0].x;   // c <= kListCap entries, unused nibbles are zero
             uint32_t seen = own;
-            const int nq = p.ns + p.ng;
-            for (int q = 0; q < nq && !over; q++)
+            if (NS != 27)
             {
-                const signed char* d = q < p.ns ? p.lap_d[q] : p.grad_d[q - p.ns];
-                const int pl = d[0] < 0 ? sl0 : (d[0] > 0 ? sl2 : sl1);
-                const int r = rec0 + d[1] * kC + d[2];
-                const uint32_t fresh = S.word[pl][r] & 0xFFFFu & ~seen;
-                if (fresh) append_fresh(S, pl, r, fresh, ls, n, over);
-                seen |= fresh;
+                // 7-point Laplacian: its neighbours first, then the gradient pass over all 26
+                const uint32_t face[6] = {mid0, S.word[sl1][rec0 - kC], S.word[sl1][rec0 - 1],
+                                          S.word[sl1][rec0 + 1], S.word[sl1][rec0 + kC], mid2};
+#pragma unroll
+                for (int q = 0; q < 6; q++)
+                {
+                    const uint32_t fresh = face[q] & 0xFFFFu & ~seen;
+                    if (fresh)
+                        append_fresh(S, q == 0 ? sl0 : (q == 5 ? sl2 : sl1),
+                                     rec0 + (q == 1 ? -kC : (q == 2 ? -1 : (q == 3 ? 1 : (q == 4 ? kC : 0)))), fresh, ls, n);
+                    seen |= fresh;
+                }
             }
+            if (NS == 27 || p.ng > 0)
+            {
+#pragma unroll
+                for (int q = 0; q < 9; q++)
+                {
+                    const uint32_t w = q < 3 ? row0[q] : (q < 6 ? row1[q - 3] : row2[q - 6]);
+                    const uint32_t fresh = w & 0xFFFFu & ~seen;
+                    if (fresh == 0u) continue;
+                    if ((fresh & (fresh - 1u)) == 0u)
+                    {
+                        ls |= (uint32_t)(__ffs(fresh) - 1) << ((4 * n) & 31);
+                        n++;
+                    }
+                    else
+                    {
+                        // several in one row: in the order of its records
+                        uint32_t left = fresh;
+                        for (int dz = -1; dz <= 1; dz++)
+                        {
+                            const int pl = q < 3 ? sl0 : (q < 6 ? sl1 : sl2);
+                            const int r = rec0 + (q - (q < 3 ? 1 : (q < 6 ? 4 : 7))) * kC + dz;
+                            const uint32_t f = S.word[pl][r] & left;
+                            if (f) append_fresh(S, pl, r, f, ls, n);
+                            left &= ~f;
+                        }
+                    }
+                    seen |= fresh;
+                }
+            }
+            over = n > kListCap;
         }
         if (over || n < 2)
         {
