@@ -34,6 +34,12 @@ __device__ __forceinline__ int pair_pos(int a, int b, int n)
 __device__ __forceinline__ double dmax_ref(double a, double b) { return (a < b) ? b : a; }  // std::max
 __device__ __forceinline__ double dmin_ref(double a, double b) { return (b < a) ? b : a; }  // std::min
 
+// Index of the phase pair of two grains (one phase: no grain's phase is looked up).
+__device__ __forceinline__ int phase_pair(const StepParams& p, const StepArrays& a, int ga, int gb)
+{
+    return p.nphases == 1 ? 0 : a.gphase[ga] * p.nphases + a.gphase[gb];
+}
+
 __device__ __forceinline__ double pair_energy(const StepParams& p, const StepArrays& a, int ga, int gb)
 {
     if (p.pair_mode == 1 && a.pair_sigma) return a.pair_sigma[(long long)ga * p.ngrains + gb];
@@ -42,13 +48,13 @@ __device__ __forceinline__ double pair_energy(const StepParams& p, const StepArr
         const unsigned long long lo = ga < gb ? ga : gb, hi = ga < gb ? gb : ga;
         return p.hash_lo + p.hash_span * uniform01(p.hash_seed, kStreamSigma, lo, hi);
     }
-    return p.sigma_p[a.gphase[ga] * p.nphases + a.gphase[gb]];
+    return p.sigma_p[phase_pair(p, a, ga, gb)];
 }
 
 __device__ __forceinline__ double pair_mobility(const StepParams& p, const StepArrays& a, int ga, int gb)
 {
     if (p.pair_mode == 1 && a.pair_mu) return a.pair_mu[(long long)ga * p.ngrains + gb];
-    return p.mu_p[a.gphase[ga] * p.nphases + a.gphase[gb]];
+    return p.mu_p[phase_pair(p, a, ga, gb)];
 }
 
 // The driving force of a grain pair after the tanh limiter (src/DrivingForce.cpp:548-583):

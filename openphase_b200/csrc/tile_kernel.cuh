@@ -664,6 +664,12 @@ constexpr int kVolCache = 4;       // per-thread grain-volume cache of the compu
 // range (bucket_off); each CUDA block takes an equal contiguous part of it, its warps 32
 // consecutive entries at a time, so that no warp idles while another drains a long slice.
 //
+// Bound: issue and latency at 16-20 warps per SM -- FP64 arithmetic, pair-table loads and, for long
+// lists, instruction fetch -- not bandwidth (N = 4 at 256^3: 0.45 ms for 0.09 ms of traffic).  Leaving
+// out what repeats (one sum per field instead of one per pair and third field, one pass for merge and
+// plausibility, no limits where no field leaves [0, 1]) took N = 2..8 at 256^3, FP64, from 235 443 519
+// 396 283 185 147 us to 235 391 452 305 219 131 129.
+//
 // N <= kListCap <= the stored fields per voxel, so a new record always fits.  AVG: averaged driving
 // forces (a template parameter: the mask costs the plain step registers).
 template <class R, int N, bool AVG>
@@ -730,18 +736,14 @@ __global__ void __launch_bounds__(128) list_compute_kernel(const __grid_constant
             lap[k] = rv[N + k];
         }
         // ---- pair kinetics ---------------------------------------------------------------------
-        double localN;
-        if (p.consider_nucleus_volume)
-        {
-            localN = 0.0;
+        double vr[N];
+        bool full = true;   // every grain at its reference volume (VolumeRatio 1)
 #pragma unroll
-            for (int k = 0; k < N; k++) localN += a.vr[g[k]];
-        }
-        else
+        for (int k = 0; k < N; k++)
         {
-            localN = (double)N;
+            vr[k] = a.vr[g[k]];
+            full = full && vr[k] == 1.0;
         }
-        const R norm_1 = (R)(1.0 / localN);
         R sg[NP];
 #pragma unroll
         for (int i = 0; i < N; i++)
@@ -749,39 +751,82 @@ __global__ void __launch_bounds__(128) list_compute_kernel(const __grid_constant
             for (int j = i + 1; j < N; j++) sg[pair_pos(i, j, N)] = (R)pair_energy(p, a, g[i], g[j]);
         const R pref = (R)p.pref_do;
         double pv[NP];
+        if (full && p.tj_factor == 0.0)
+        {
+            // The usual case.  With every scale 1 the factor h is one number (R(0.5) * (R(1) + R(1)) *
+            // pref = pref), so lap + h*val is formed once per field instead of once per pair and third
+            // field, the triple-junction term is absent and LocalN = N: the same operations on the
+            // same operands as below, without their repetitions.
+            const R norm_1 = (R)(1.0 / (double)N);
+            R sum[N];
 #pragma unroll
-        for (int i = 0; i < N; i++)
+            for (int k = 0; k < N; k++) sum[k] = lap[k] + pref * val[k];
 #pragma unroll
-            for (int j = i + 1; j < N; j++)
-            {
-                const int q = pair_pos(i, j, N);
-                const double vri = a.vr[g[i]], vrj = a.vr[g[j]];
-                const R scale = (vri == 1.0 && vrj == 1.0) ? R(1) : (R)sqrt(vri * vrj);
-                const R h = R(0.5) * (R(1) + scale) * pref;
-                R dphi = sg[q] * ((lap[i] + h * val[i]) - (lap[j] + h * val[j]));
-                if (N > 2)
+            for (int i = 0; i < N; i++)
+#pragma unroll
+                for (int j = i + 1; j < N; j++)
                 {
+                    const int q = pair_pos(i, j, N);
+                    R dphi = sg[q] * (sum[i] - sum[j]);
 #pragma unroll
                     for (int k = 0; k < N; k++)
                     {
                         if (k == i || k == j) continue;
                         const R sbk = sg[j < k ? pair_pos(j, k, N) : pair_pos(k, j, N)];
                         const R sak = sg[i < k ? pair_pos(i, k, N) : pair_pos(k, i, N)];
-                        dphi += (sbk - sak) * (lap[k] + h * val[k]);
-                        if (p.tj_factor != 0.0 || scale < R(1))
+                        dphi += (sbk - sak) * sum[k];
+                    }
+                    dphi *= (R)pair_mobility(p, a, g[i], g[j]) * norm_1;
+                    pv[q] = (double)dphi;
+                }
+        }
+        else
+        {
+            double localN;
+            if (p.consider_nucleus_volume)
+            {
+                localN = 0.0;
+#pragma unroll
+                for (int k = 0; k < N; k++) localN += vr[k];
+            }
+            else
+            {
+                localN = (double)N;
+            }
+            const R norm_1 = (R)(1.0 / localN);
+#pragma unroll
+            for (int i = 0; i < N; i++)
+#pragma unroll
+                for (int j = i + 1; j < N; j++)
+                {
+                    const int q = pair_pos(i, j, N);
+                    const R scale = (vr[i] == 1.0 && vr[j] == 1.0) ? R(1) : (R)sqrt(vr[i] * vr[j]);
+                    const R h = R(0.5) * (R(1) + scale) * pref;
+                    R dphi = sg[q] * ((lap[i] + h * val[i]) - (lap[j] + h * val[j]));
+                    if (N > 2)
+                    {
+#pragma unroll
+                        for (int k = 0; k < N; k++)
                         {
-                            const int pA = a.gphase[g[i]], pB = a.gphase[g[j]], pG = a.gphase[g[k]];
-                            const int P = p.nphases;
-                            const R tj = (R)dmax_ref(p.tj_factor, (double)(R(1) - scale));
-                            dphi += tj * pref
-                                  * (((R)p.sigma_p[pA * P + pB] + (R)p.sigma_p[pB * P + pG]) + (R)p.sigma_p[pA * P + pG])
-                                  * (val[i] * val[k] - val[j] * val[k]);
+                            if (k == i || k == j) continue;
+                            const R sbk = sg[j < k ? pair_pos(j, k, N) : pair_pos(k, j, N)];
+                            const R sak = sg[i < k ? pair_pos(i, k, N) : pair_pos(k, i, N)];
+                            dphi += (sbk - sak) * (lap[k] + h * val[k]);
+                            if (p.tj_factor != 0.0 || scale < R(1))
+                            {
+                                const int pA = a.gphase[g[i]], pB = a.gphase[g[j]], pG = a.gphase[g[k]];
+                                const int P = p.nphases;
+                                const R tj = (R)dmax_ref(p.tj_factor, (double)(R(1) - scale));
+                                dphi += tj * pref
+                                      * (((R)p.sigma_p[pA * P + pB] + (R)p.sigma_p[pB * P + pG]) + (R)p.sigma_p[pA * P + pG])
+                                      * (val[i] * val[k] - val[j] * val[k]);
+                            }
                         }
                     }
+                    dphi *= (R)pair_mobility(p, a, g[i], g[j]) * norm_1 * scale;
+                    pv[q] = (double)dphi;
                 }
-                dphi *= (R)pair_mobility(p, a, g[i], g[j]) * norm_1 * scale;
-                pv[q] = (double)dphi;
-            }
+        }
         // ---- driving force (interface voxels only) ----------------------------------------------
         if (p.use_dg && flag == 2)
         {
@@ -807,9 +852,10 @@ __global__ void __launch_bounds__(128) list_compute_kernel(const __grid_constant
         }
         // ---- projection ---------------------------------------------------------------------------
         const double dt = p.dt;
+        bool any = false;   // lists of more than two fields: some increment is left
         if (NP == 1)
         {
-            const double valueA = (pv[0] + 0.0) * dt;
+            const double valueA = pv[0] * dt;
             const double old_value = (double)val[0];
             if ((old_value == 0.0 && valueA < 0.0) || (old_value == 1.0 && valueA > 0.0))
             {
@@ -830,6 +876,7 @@ __global__ void __launch_bounds__(128) list_compute_kernel(const __grid_constant
 #pragma unroll
             for (int i = 0; i < N; i++)
             {
+                if (val[i] != R(0) && val[i] != R(1)) continue;   // the sum is read at a bound only
                 double dpsi = 0.0;
 #pragma unroll
                 for (int j = 0; j < N; j++)
@@ -837,7 +884,7 @@ __global__ void __launch_bounds__(128) list_compute_kernel(const __grid_constant
                     if (j == i) continue;
                     dpsi += (i < j) ? pv[pair_pos(i, j, N)] : pv[pair_pos(j, i, N)] * (-1.0);
                 }
-                if (((double)val[i] == 0.0 && dpsi < 0.0) || ((double)val[i] == 1.0 && dpsi > 0.0))
+                if ((val[i] == R(0) && dpsi < 0.0) || (val[i] == R(1) && dpsi > 0.0))
                 {
 #pragma unroll
                     for (int j = 0; j < N; j++)
@@ -847,7 +894,6 @@ __global__ void __launch_bounds__(128) list_compute_kernel(const __grid_constant
                     }
                 }
             }
-            bool any = false;
 #pragma unroll
             for (int q = 0; q < NP; q++) any |= (pv[q] != 0.0);
             if (any)
@@ -866,17 +912,19 @@ __global__ void __launch_bounds__(128) list_compute_kernel(const __grid_constant
                             if (w < 0.0) { neg[i] += w; pos[j] += -w; }
                             if (w > 0.0) { pos[i] += w; neg[j] += -w; }
                         }
+                    bool outside = false;
 #pragma unroll
                     for (int i = 0; i < N; i++)
                     {
                         const double vi = (double)val[i];
                         const double newPF = vi + (pos[i] + neg[i]) * dt;
                         double limN = 1.0, limP = 1.0;
-                        if (newPF < 0.0) limN = dmin_ref(1.0, -(vi + pos[i] * dt) / (neg[i] * dt));
-                        if (newPF > 1.0) limP = dmin_ref(1.0, (1.0 - (vi + neg[i] * dt)) / (pos[i] * dt));
+                        if (newPF < 0.0) { outside = true; limN = dmin_ref(1.0, -(vi + pos[i] * dt) / (neg[i] * dt)); }
+                        if (newPF > 1.0) { outside = true; limP = dmin_ref(1.0, (1.0 - (vi + neg[i] * dt)) / (pos[i] * dt)); }
                         neg[i] = limN;
                         pos[i] = limP;
                     }
+                    if (!outside) break;   // every limit is 1
                     bool needed = false;
 #pragma unroll
                     for (int i = 0; i < N; i++)
@@ -900,26 +948,12 @@ __global__ void __launch_bounds__(128) list_compute_kernel(const __grid_constant
                     if (!needed) break;
                     if (it == 25) st |= kStLimiterCap;
                 }
-#pragma unroll
-                for (int q = 0; q < NP; q++)
-                    if (fabs(pv[q] * dt) < DBL_EPSILON) pv[q] = 0.0;
-                double chk[N];
-#pragma unroll
-                for (int i = 0; i < N; i++) chk[i] = (double)val[i];
-#pragma unroll
-                for (int i = 0; i < N; i++)
-#pragma unroll
-                    for (int j = i + 1; j < N; j++)
-                    {
-                        const double w = pv[pair_pos(i, j, N)];
-                        if (w != 0.0) { chk[i] += w * dt; chk[j] += -w * dt; }
-                    }
-#pragma unroll
-                for (int i = 0; i < N; i++)
-                    if (chk[i] < -(double)FLT_EPSILON || chk[i] > 1.0 + (double)FLT_EPSILON) st |= kStNormalizeWarn;
             }
         }
         // ---- merge (FP64) and finalize --------------------------------------------------------------
+        // The reference first zeroes the increments below DBL_EPSILON, then tries them for plausibility
+        // (a warning) and then merges those of at least DBL_EPSILON: one pass, since both sums have the
+        // same terms in the same order.
         double vd[N];
 #pragma unroll
         for (int i = 0; i < N; i++) vd[i] = (double)val[i];
@@ -928,13 +962,19 @@ __global__ void __launch_bounds__(128) list_compute_kernel(const __grid_constant
 #pragma unroll
             for (int j = i + 1; j < N; j++)
             {
-                const double value = 1.0 * (pv[pair_pos(i, j, N)] + 0.0) * dt;
+                const double value = pv[pair_pos(i, j, N)] * dt;
                 if (fabs(value) >= DBL_EPSILON)
                 {
                     vd[i] += value;
                     vd[j] += -value;
                 }
             }
+        if (any)
+        {
+#pragma unroll
+            for (int i = 0; i < N; i++)
+                if (vd[i] < -(double)FLT_EPSILON || vd[i] > 1.0 + (double)FLT_EPSILON) st |= kStNormalizeWarn;
+        }
         const double hi_snap = 1.0 - p.eps_snap;
         const double lo_snap = 0.0 + p.eps_snap;
         double total = 0.0;
