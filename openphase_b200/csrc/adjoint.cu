@@ -999,7 +999,7 @@ adjoint_gather_kernel(const __grid_constant__ StepParams p, const StepArrays la,
     const int z = z0 + tz, y = y0 + ty;
     const bool inside = (z < nz) && (y < ny);
 
-    for (int i = t; i < kSlots * 3 * Geo::kRecs; i += NT) (&S.dense[0][0][0])[i] = 0.0;
+    for (int i = t; i < (int)(sizeof(S.dense) / sizeof(double)); i += NT) reinterpret_cast<double*>(S.dense)[i] = 0.0;
     for (int i = t; i < 3 * Geo::kRecs; i += NT) (&S.word[0][0])[i] = 0u;
     if (t < 16) { S.grain_of[t] = -1; S.lastpos[t] = -1000; }
     for (int i = t; i < kSlotMap; i += NT) S.map[i] = 0;
@@ -1052,7 +1052,7 @@ adjoint_gather_kernel(const __grid_constant__ StepParams p, const StepArrays la,
                         const int dx = stencil_dx<NS>(q);
                         const int pl = dx > 0 ? sl0 : (dx < 0 ? sl2 : sl1);
                         const int r = rec0 - stencil_dy<NS>(q) * kC - stencil_dz<NS>(q);
-                        l += p.lap_w[q] * S.dense[k][pl][r];
+                        l += p.lap_w[q] * S.dense[k].at[pl][r];
                     }
                 }
             }

@@ -103,8 +103,8 @@ def test_averaging_dense_and_wrapped_grids(name, variant):
 @pytest.mark.parametrize("precision", ["fp64", "fp32"])
 @pytest.mark.parametrize("threshold", [0.0, 0.02])
 def test_averaging_tiled_equals_generic(precision, threshold):
-    """Both kernels read the same mask: large grains (VolumeRatio = 1) give identical lists in either
-    precision, the FP64 values bit for bit; a low threshold makes most marks "several"."""
+    """Both kernels read the same mask: large grains (VolumeRatio = 1) give identical lists and values
+    bit for bit; a low threshold makes most marks "several"."""
     case = Case(40, 33, 37, 10, seed=19, iwidth=5.0, dt=0.08, dg_scale=0.1, average=True, name="tiled_generic")
     state = case.initial_state()
     got = []
@@ -115,7 +115,4 @@ def test_averaging_tiled_equals_generic(precision, threshold):
         ctx.step(case.dt, 3)
         got.append(ctx.download())
     r = compare_states(*got, case.ngrains)
-    if precision == "fp64":
-        assert r["same_sets"] and r["max_dphi"] == 0.0, r
-    else:
-        assert r["max_dphi"] <= 1e-3, r   # FP32 Laplacians are fused in one and not in the other
+    assert r["same_sets"] and r["max_dphi"] == 0.0, r

@@ -15,6 +15,7 @@ from openphase_b200._lib import OpgpuError
 from openphase_b200.cases import Case
 from openphase_b200.context import Context
 from oracle.bridge import Oracle
+from tests.golden.make_golden import GOLDEN_CASES
 from tests.parity import compare_states
 
 pytestmark = pytest.mark.gpu
@@ -126,3 +127,26 @@ def test_step_timing_on_every_path(aniso):
     assert 0.0 <= s["timed_classify_ms"] <= s["timed_kernel_ms"]
     if aniso:
         assert s["timed_classify_ms"] < 0.1 * s["timed_kernel_ms"]
+
+
+ANISO = [n for n in GOLDEN_CASES if GOLDEN_CASES[n][0].phase_cubic_eps is not None]
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("name", ANISO)
+def test_anisotropic_lists_equal_generic_kernel(name, precision):
+    """Anisotropic set-ups on the classified lists against the full-grid generic kernel: the same lists,
+    counts and values up to the grain volumes' summation order (VolumeRatio < 1 here; in FP32 a last-bit
+    difference of a ratio is below the rounding of the values)."""
+    case, _ = GOLDEN_CASES[name]
+    state = case.initial_state()
+    got = []
+    for variant in ("tiled", "generic"):
+        ctx = Context.from_case(case, precision=precision, k_slots=16, state=state)
+        ctx.set_kernel_variant(variant)
+        assert ctx.step(case.dt, 6) & 0b11 == 0
+        got.append((ctx.download(), ctx.stats()))
+    r = compare_states(got[0][0], got[1][0], case.ngrains)
+    assert r["same_sets"] and r["max_dphi"] <= (1e-12 if precision == "fp64" else 1e-6), r
+    for key in ("wide_total", "entries_in_total", "entries_out_total"):
+        assert got[0][1][key] == got[1][1][key], key
