@@ -986,7 +986,6 @@ adjoint_gather_kernel(const __grid_constant__ StepParams p, const StepArrays la,
     using Smem = TileSmem<double, TY>;
     constexpr int NT = Geo::NT;
     constexpr int kC = Geo::kCols;
-    constexpr int kSlots = WindowSlots<double>::value;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Smem& S = *reinterpret_cast<Smem*>(smem_raw);
 

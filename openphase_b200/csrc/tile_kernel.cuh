@@ -98,9 +98,13 @@ __device__ __forceinline__ unsigned slot_hash(int g) { return ((unsigned)g * 265
 // and add (the FP64 unit is compiled without contraction).  FP32: one fused multiply-add, written
 // out because the FP32 unit is compiled without contraction too (so that the adjoint can repeat its
 // per-voxel arithmetic exactly); these Laplacians reach the forward and the adjoint alike through
-// the work records, so their rounding only has to be the same in both, which it is.
+// the work records, so their rounding only has to be the same in both, which it is.  Steps with
+// anisotropic models or averaged driving forces (no adjoint) keep the separate operations of the
+// generic kernel in either precision (FUSED = false).
+template <bool FUSED>
 __device__ __forceinline__ double lap_acc(double l, double w, double x) { return l + w * x; }
-__device__ __forceinline__ float lap_acc(float l, float w, float x) { return __fmaf_rn(w, x, l); }
+template <bool FUSED>
+__device__ __forceinline__ float lap_acc(float l, float w, float x) { return FUSED ? __fmaf_rn(w, x, l) : l + w * x; }
 
 // Slot of a grain in the window (-1 if the grain has none).  A window holds at most 16 grains, so
 // the map hits but for a few per cent of the grains, whose entry another grain of the window took;
@@ -405,7 +409,7 @@ __device__ __forceinline__ void append_fresh(const TileSmem<R, TY>& S, int pl, i
     }
 }
 
-template <class R, int TY, int NS>
+template <class R, int TY, int NS, bool FUSED>
 __global__ void __launch_bounds__(kTileZ * TY, sizeof(R) == 8 ? 3 : 5)
 tile_classify_kernel(const __grid_constant__ StepParams p, const StepArrays a, int xchunk)
 {
@@ -431,7 +435,6 @@ tile_classify_kernel(const __grid_constant__ StepParams p, const StepArrays a, i
     R* __restrict__ vout = static_cast<R*>(a.val_out);
 
     for (int i = t; i < kClassifyVolSlots; i += NT) { S.vol_key[i] = -1; S.vol_sum[i] = 0.0; }
-    constexpr int kSlots = WindowSlots<R>::value;
     for (int i = t; i < (int)(sizeof(S.dense) / sizeof(R)); i += NT) reinterpret_cast<R*>(S.dense)[i] = R(0);
     for (int i = t; i < 3 * Geo::kRecs; i += NT) (&S.word[0][0])[i] = 0u;
     if (t < 16) { S.grain_of[t] = -1; S.lastpos[t] = -1000; }
@@ -609,7 +612,7 @@ tile_classify_kernel(const __grid_constant__ StepParams p, const StepArrays a, i
                 const int dx = stencil_dx<NS>(q);
                 const int pl = dx < 0 ? sl0 : (dx > 0 ? sl2 : sl1);
                 const int r = rec0 + stencil_dy<NS>(q) * kC + stencil_dz<NS>(q);
-                l = lap_acc(l, (R)p.lap_w[q], S.dense[s].at[pl][r]);
+                l = lap_acc<FUSED>(l, (R)p.lap_w[q], S.dense[s].at[pl][r]);
             }
             rg[k] = (int16_t)S.grain_of[s];
             rv[k] = S.dense[s].at[sl1][rec0];
@@ -1041,6 +1044,128 @@ __global__ void __launch_bounds__(128) list_compute_kernel(const __grid_constant
     flush_block(a, 0u, 0u, eout, st, s_cnt, s_key, s_sum, kTileVolSlots, t, blockDim.x);
 }
 
+// ---- anisotropic energies and mobilities -----------------------------------------------------------
+// Neighbour of a voxel at offset d without indexing the offset arrays by a runtime value.
+__device__ __forceinline__ long long nb_at(const Neighbourhood& nb, const signed char* d)
+{
+    const long long x = d[0] < 0 ? nb.X[0] : (d[0] > 0 ? nb.X[2] : nb.X[1]);
+    const long long y = d[1] < 0 ? nb.Y[0] : (d[1] > 0 ? nb.Y[2] : nb.Y[1]);
+    const long long z = d[2] < 0 ? nb.Z[0] : (d[2] > 0 ? nb.Z[2] : nb.Z[1]);
+    return x + y + z;
+}
+
+// Models of the interface normal need the gradient of every list entry besides the classify kernel's
+// list, values and Laplacians.  One thread per wide voxel of list length blockIdx.y + 2: the
+// gradients from the neighbours in global memory, in gradient-stencil order as gather_list sums them,
+// then list_step with its working arrays (capacity kListCap) in local memory.  Bound: the latency of
+// the neighbour loads and of the model functions (pow, acos); in an early solidification one voxel in
+// ten is wide, so a warp over the wide voxels instead of over the grid has ten times the lanes at
+// work, and the bulk voxels cost the classify kernel's copy only.
+template <class R>
+__global__ void __launch_bounds__(128) aniso_list_kernel(const __grid_constant__ StepParams p, const StepArrays a,
+                                                         int nslices)
+{
+    __shared__ int s_key[kTileVolSlots];
+    __shared__ double s_sum[kTileVolSlots];
+    __shared__ unsigned long long s_cnt[3];
+    const int n = blockIdx.y + 2, t = threadIdx.x;
+    const unsigned* __restrict__ off = a.bucket_off + (long long)n * (nslices + 1);
+    const unsigned total = off[nslices];
+    const unsigned per = ((total + gridDim.x * blockDim.x - 1u) / (gridDim.x * blockDim.x)) * blockDim.x;
+    const unsigned r0 = blockIdx.x * per;
+    if (r0 >= total) return;
+    const unsigned r1 = min(total, r0 + per);
+    for (int i = t; i < kTileVolSlots; i += blockDim.x) { s_key[i] = -1; s_sum[i] = 0.0; }
+    if (t < 3) s_cnt[t] = 0ull;
+    __syncthreads();
+    const long long N = p.n;
+    const uint8_t* __restrict__ cnt = a.cnt_in;
+    const int16_t* __restrict__ gin = a.idx_in;
+    const R* __restrict__ vin = static_cast<const R*>(a.val_in);
+    R* __restrict__ vout = static_cast<R*>(a.val_out);
+    const int2* __restrict__ buck = a.bucket + (long long)n * a.bucket_cap;
+    const int pad = ((2 * n + 7) / 8) * 8;
+    uint32_t st = 0;
+    unsigned eout = 0;
+    for (unsigned e = r0 + t; e < r1; e += blockDim.x)
+    {
+        const int sl = slice_of(off, nslices, e);
+        const int2 ent = buck[(long long)sl * a.slice + (e - off[sl])];
+        const unsigned char* __restrict__ wbase = a.wl + (long long)sl * a.wl_slice + ent.y;
+        const long long v = ent.x & 0x7fffffff;
+        const int flag = (ent.x >> 31) ? 2 : 1;
+        const int16_t* __restrict__ rg = reinterpret_cast<const int16_t*>(wbase);
+        const R* __restrict__ rv = reinterpret_cast<const R*>(wbase + pad);
+        constexpr int KP = kListCap * (kListCap - 1) / 2;
+        int16_t g[kListCap];
+        R val[kListCap], lap[kListCap], sg[KP], grad[3 * kListCap];
+        double pv[KP], pos[kListCap], neg[kListCap];
+        for (int k = 0; k < n; k++)
+        {
+            g[k] = rg[k];
+            val[k] = rv[k];
+            lap[k] = rv[n + k];
+            grad[3 * k] = grad[3 * k + 1] = grad[3 * k + 2] = R(0);
+        }
+        const Neighbourhood nb(p, v);
+        for (int q = 0; q < p.ngs; q++)
+        {
+            const long long u = nb_at(nb, p.gs_d[q]);
+            const int cu = cnt[u];
+            for (int s = 0; s < cu; s++)
+            {
+                const R phi = vin[s * N + u];
+                const int gu = gin[s * N + u];
+                int f = 0;
+                while (f < n && g[f] != gu) f++;
+                if (f < n)
+                {
+                    const R gx = (R)p.gs_w[q][0] * phi;
+                    const R gy = (R)p.gs_w[q][1] * phi;
+                    const R gz = (R)p.gs_w[q][2] * phi;
+                    grad[3 * f] += gx;
+                    grad[3 * f + 1] += gy;
+                    grad[3 * f + 2] += gz;
+                }
+            }
+        }
+        const ListScratch<R> sc{g, val, lap, sg, pv, pos, neg, 1, grad};
+        const int m = list_step<R>(p, a, sc, n, flag, st, v, (int)cnt[v]);
+        a.cnt_out[v] = (uint8_t)m;
+        for (int i = 0; i < m; i++)
+        {
+            a.idx_out[i * N + v] = g[i];
+            vout[i * N + v] = val[i];
+            if (in_volume_window(p, v)) vol_insert_n(s_key, s_sum, kTileVolSlots, a.vol_acc, g[i], (double)val[i]);
+        }
+        eout += m;
+    }
+    flush_block(a, 0u, 0u, eout, st, s_cnt, s_key, s_sum, kTileVolSlots, t, blockDim.x);
+}
+
+// The general-path worklist with anisotropic models: one thread per voxel.
+template <class R, int KS, int KL>
+__global__ void __launch_bounds__(64) aniso_worklist_kernel(const __grid_constant__ StepParams p, const StepArrays a)
+{
+    __shared__ int s_key[kTileVolSlots];
+    __shared__ double s_sum[kTileVolSlots];
+    __shared__ unsigned long long s_cnt[3];
+    for (int i = threadIdx.x; i < kTileVolSlots; i += blockDim.x) { s_key[i] = -1; s_sum[i] = 0.0; }
+    if (threadIdx.x < 3) s_cnt[threadIdx.x] = 0ull;
+    __syncthreads();
+    const unsigned total = min(*a.slow_count, a.slow_cap);
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&a.counters[kCntGeneralLast], (unsigned long long)total);
+    uint32_t st = 0;
+    unsigned eo = 0;
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x)
+    {
+        unsigned wide = 0, ein = 0, eout = 0;   // wide and ein were counted by the classify kernel
+        voxel_step_generic<R, KS, KL, true>(p, a, a.slow_list[i], s_key, s_sum, kTileVolSlots, wide, ein, eout, st, false);
+        eo += eout;
+    }
+    flush_block(a, 0u, 0u, eo, st, s_cnt, s_key, s_sum, kTileVolSlots, threadIdx.x, blockDim.x);
+}
+
 // Fork of the side streams from a context's stream, and their join into it.  join() is called on
 // every path that launched on them, so that no work of a step outlives the step's place in the
 // context's stream.
@@ -1101,30 +1226,41 @@ int launch_tiled_ns(const StepParams& p, const StepArrays& a, void* stream, Laun
     int xchunk = 0, gz = 0, gy = 0, gx = 0;
     tiled_geometry(p.nx, p.ny, p.nz, &xchunk, &gz, &gy, &gx);
     const int nblocks = gz * gy * gx;
-    auto kern = tile_classify_kernel<R, kTileTY, NS>;
+    constexpr bool kSingle = sizeof(R) == 4;
+    auto kern = kSingle && !p.aniso && !a.avg_mask ? tile_classify_kernel<R, kTileTY, NS, kSingle>
+                                                  : tile_classify_kernel<R, kTileTY, NS, false>;
     const size_t smem = sizeof(Smem);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+    auto gk = warp_general_kernel<R, KS, KL>;
+    const size_t wsm = 4 * sizeof(WarpScratch<R, KL>);
+    e = cudaFuncSetAttribute(gk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wsm);
     if (e != cudaSuccess) return (int)e;
     e = cudaMemsetAsync(a.slow_count, 0, sizeof(unsigned), s);
     if (e != cudaSuccess) return (int)e;
     kern<<<dim3(gz, gy, gx), dim3(kTileZ, kTileTY), smem, s>>>(p, a, xchunk);
-    if (info && info->after_classify)
+    // (anisotropic steps report no classify share: their timing is that of the whole step)
+    if (info && info->after_classify && !p.aniso)
     {
         e = cudaEventRecord(static_cast<cudaEvent_t>(info->after_classify), s);
         if (e != cudaSuccess) return (int)e;
     }
     bucket_scan_kernel<<<kListCap - 1, 1024, 0, s>>>(a, nblocks);
     const int cb = compute_blocks(p.n);
-    auto gk = warp_general_kernel<R, KS, KL>;
-    const size_t wsm = 4 * sizeof(WarpScratch<R, KL>);
-    e = cudaFuncSetAttribute(gk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wsm);
-    if (e != cudaSuccess) return (int)e;
     const SideFork fork(info && p.n <= kSideVoxels ? info->side : nullptr, s);
-    gk<<<148 * 4, 128, wsm, fork.on(2)>>>(p, a);
-    if (a.avg_mask) launch_lists<R, true>(p, a, cb, nblocks, fork);
-    else launch_lists<R, false>(p, a, cb, nblocks, fork);
+    if (p.aniso)
+    {
+        aniso_worklist_kernel<R, KS, KL><<<148 * 8, 64, 0, fork.on(0)>>>(p, a);
+        aniso_list_kernel<R><<<dim3(cb, kListCap - 1), 128, 0, s>>>(p, a, nblocks);
+    }
+    else
+    {
+        gk<<<148 * 4, 128, wsm, fork.on(2)>>>(p, a);
+        if (a.avg_mask) launch_lists<R, true>(p, a, cb, nblocks, fork);
+        else launch_lists<R, false>(p, a, cb, nblocks, fork);
+    }
     if ((e = fork.join()) != cudaSuccess) return (int)e;
-    if (info) info->kernels += 10;
+    if (info) info->kernels += p.aniso ? 4 : 10;
     return (int)cudaGetLastError();
 }
 
@@ -1138,7 +1274,7 @@ int launch_classify_ns(const StepParams& p, const StepArrays& a, void* stream)
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     int xchunk = 0, gz = 0, gy = 0, gx = 0;
     tiled_geometry(p.nx, p.ny, p.nz, &xchunk, &gz, &gy, &gx);
-    auto kern = tile_classify_kernel<R, kTileTY, NS>;
+    auto kern = tile_classify_kernel<R, kTileTY, NS, sizeof(R) == 4>;
     const size_t smem = sizeof(Smem);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return -(int)e;
@@ -1168,10 +1304,8 @@ template <class R>
 int launch_step(const StepParams& p, const StepArrays& a, int k_slots, int variant, void* stream,
                 LaunchInfo* info)
 {
-    if (variant == kVariantGeneric || p.aniso)
+    if (variant == kVariantGeneric)
     {
-        // anisotropic energies need the gradients of every list entry: the per-voxel generic kernel
-        // only (the tiled kernels stay free of them)
         if (info) info->kernels += 1;
         return launch_step_generic<R>(p, a, k_slots, stream);
     }
