@@ -1065,7 +1065,7 @@ static int launch_gather_ns(const StepParams& p, const StepArrays& a, const AdjA
 {
     using Smem = TileSmem<double, kTileTY>;
     int xchunk = 0, gz = 0, gy = 0, gx = 0;
-    tiled_geometry(p.nx, p.ny, p.nz, &xchunk, &gz, &gy, &gx);
+    tiled_geometry(p.nx, p.ny, p.nz, 8, &xchunk, &gz, &gy, &gx);
     StepArrays la = a;   // the plane loader reads the lists of the Laplacian adjoints
     la.cnt_in = aa.lcnt;
     la.idx_in = aa.lidx;

@@ -568,7 +568,7 @@ extern "C" uint32_t opgpu_create(const opgpu_grid* grid, opgpu_ctx** out)
     if (dalloc(&ctx->d_slow_count, 1) != cudaSuccess) return bail(OPGPU_E_CUDA);
     {
         int xchunk = 0, gz = 0, gy = 0, gx = 0;
-        tiled_geometry(g.nx, g.ny, g.nz, &xchunk, &gz, &gy, &gx);
+        tiled_geometry(g.nx, g.ny, g.nz, (int)ctx->rsz, &xchunk, &gz, &gy, &gx);
         const long long nblocks = (long long)gz * gy * gx;
         ctx->slice = kTileCols * kTileRows * xchunk;
         ctx->bucket_cap = nblocks * ctx->slice;

@@ -156,17 +156,30 @@ constexpr int kTileCols = 16;  // tile of the classify kernel: kTileCols (z) x k
 constexpr int kTileRows = 8;   // one thread each
 
 // Launch geometry of the classify kernel: tiles of kTileCols (z) x kTileRows (y) voxels marching over
-// `xchunk` x-planes; enough x-chunks for several blocks per SM on small grids, long chunks (halo
-// reuse) on large ones.  slice = voxels one block can append to a bucket.
-inline void tiled_geometry(int nx, int ny, int nz, int* xchunk, int* gz, int* gy, int* gx)
+// `xchunk` x-planes.  A block loads xchunk + 2 planes and spends about one more on setting up its
+// shared memory; the device holds 148 SMs x 3 (FP64) or 5 (FP32) blocks at a time.  The estimate is
+// planes times waves, plus a third of a wave for blocks over bulk and over interfaces that differ in
+// length; the shortest wins.  Measured, classify in us (chunk): FP64 64^3 81 (2) 62 (5); 96^3 181 (5) 151
+// (8) 140 (16); 128^3 318 (13) 345 (16) 372 (43); 160^3 566 (15) 577 (20); FP32 150x97x203, 7-point 376
+// (15) 365 (21) 341 (38): the estimate's order each time.  slice = voxels one block can append to a
+// bucket.
+inline void tiled_geometry(int nx, int ny, int nz, int real_size, int* xchunk, int* gz, int* gy, int* gx)
 {
     const int tzb = (nz + kTileCols - 1) / kTileCols, tyb = (ny + kTileRows - 1) / kTileRows;
-    long long xc = (long long)nx * tzb * tyb / (148 * 8);
-    xc = xc < 2 ? 2 : (xc > 32 ? 32 : xc);
-    *xchunk = (int)xc;
+    const long long tiles = (long long)tzb * tyb, resident = 148 * (real_size == 8 ? 3 : 5);
+    long long best = 0;
+    int xc = 2;
+    for (int c = 2; c <= 64 && c <= nx + 1; c++)
+    {
+        const long long blocks = tiles * ((nx + c - 1) / c);
+        const long long waves = (blocks + resident - 1) / resident;
+        const long long cost = (c + 3) * (20 * waves + 7);
+        if (best == 0 || cost < best) { best = cost; xc = c; }
+    }
+    *xchunk = xc;
     *gz = tzb;
     *gy = tyb;
-    *gx = (int)((nx + xc - 1) / xc);
+    *gx = (nx + xc - 1) / xc;
 }
 
 enum { kVariantTiled = 0, kVariantGeneric = 1 };

@@ -1224,7 +1224,7 @@ int launch_tiled_ns(const StepParams& p, const StepArrays& a, void* stream, Laun
     using Smem = TileSmem<R, kTileTY>;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     int xchunk = 0, gz = 0, gy = 0, gx = 0;
-    tiled_geometry(p.nx, p.ny, p.nz, &xchunk, &gz, &gy, &gx);
+    tiled_geometry(p.nx, p.ny, p.nz, (int)sizeof(R), &xchunk, &gz, &gy, &gx);
     const int nblocks = gz * gy * gx;
     constexpr bool kSingle = sizeof(R) == 4;
     auto kern = kSingle && !p.aniso && !a.avg_mask ? tile_classify_kernel<R, kTileTY, NS, kSingle>
@@ -1273,7 +1273,7 @@ int launch_classify_ns(const StepParams& p, const StepArrays& a, void* stream)
     using Smem = TileSmem<R, kTileTY>;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     int xchunk = 0, gz = 0, gy = 0, gx = 0;
-    tiled_geometry(p.nx, p.ny, p.nz, &xchunk, &gz, &gy, &gx);
+    tiled_geometry(p.nx, p.ny, p.nz, (int)sizeof(R), &xchunk, &gz, &gy, &gx);
     auto kern = tile_classify_kernel<R, kTileTY, NS, sizeof(R) == 4>;
     const size_t smem = sizeof(Smem);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
