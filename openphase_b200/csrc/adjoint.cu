@@ -376,8 +376,9 @@ __global__ void __launch_bounds__(128) tlm_step_kernel(const __grid_constant__ S
 
 // ---- adjoint -------------------------------------------------------------------------------------
 // One limiter iteration of NormalizeIncrementsSR (src/PhaseField.cpp:1447-1519) on pv (in place).
-// Records the per-field sums and limits the reverse sweep needs.  Returns whether a limit < 1 acted.
-__device__ __forceinline__ bool limiter_iteration(int n, const double* val, double dt, double* pv, double* pos,
+// Records the per-field sums and limits the reverse sweep needs.  Returns 0 if no field leaves [0, 1]
+// (every limit is 1, pv is unchanged), 2 if a limit < 1 acted, else 1.
+__device__ __forceinline__ int limiter_iteration(int n, const double* val, double dt, double* pv, double* pos,
                                                   double* neg, double* limN, double* limP)
 {
     for (int i = 0; i < n; i++) { pos[i] = 0.0; neg[i] = 0.0; }
@@ -388,15 +389,18 @@ __device__ __forceinline__ bool limiter_iteration(int n, const double* val, doub
             if (w < 0.0) { neg[i] += w; pos[j] += -w; }
             if (w > 0.0) { pos[i] += w; neg[j] += -w; }
         }
+    bool outside = false;
     for (int i = 0; i < n; i++)
     {
         const double vi = val[i], pi = pos[i], ni = neg[i];
         const double newPF = vi + (pi + ni) * dt;
         limN[i] = 1.0;
         limP[i] = 1.0;
+        outside = outside || newPF < 0.0 || newPF > 1.0;
         if (newPF < 0.0) limN[i] = dmin_ref(1.0, -(vi + pi * dt) / (ni * dt));
         if (newPF > 1.0) limP[i] = dmin_ref(1.0, (1.0 - (vi + ni * dt)) / (pi * dt));
     }
+    if (!outside) return 0;
     bool needed = false;
     for (int i = 0; i < n; i++)
         for (int j = i + 1; j < n; j++)
@@ -417,7 +421,7 @@ __device__ __forceinline__ bool limiter_iteration(int n, const double* val, doub
             }
             pv[q] = w;
         }
-    return needed;
+    return needed ? 2 : 1;
 }
 
 // Sums and limits of one limiter iteration for the increments pv (pv itself is not changed).
@@ -541,11 +545,21 @@ __device__ __forceinline__ void adjoint_core(const StepParams& p, const StepArra
     const int np = n * (n - 1) / 2;
     const double dt = p.dt;
     // ---- forward recompute: pair kinetics (list_step order) ----
+    // `plain`: every grain at its reference volume and no triple-junction term, the usual case.  Then
+    // lap + h*val is one number per field, and (as in list_compute_kernel) the increments are the same
+    // operations on the same operands without their repetitions.
+    double vr[KL], sg[KP], mob[KP];
+    bool plain = p.tj_factor == 0.0;
+    for (int k = 0; k < n; k++)
+    {
+        vr[k] = a.vr[g[k]];
+        plain = plain && vr[k] == 1.0;
+    }
     double localN;
     if (p.consider_nucleus_volume)
     {
         localN = 0.0;
-        for (int k = 0; k < n; k++) localN += a.vr[g[k]];
+        for (int k = 0; k < n; k++) localN += vr[k];
     }
     else
     {
@@ -554,45 +568,74 @@ __device__ __forceinline__ void adjoint_core(const StepParams& p, const StepArra
     const double norm_1 = 1.0 / localN;
     const double pref = p.pref_do;
     double psi[KP], pv0[KP], pv[KP], lpv[KP], lpw[KP];
+    for (int i = 0; i < n; i++)
+        for (int j = i + 1; j < n; j++)
+        {
+            const int q = pair_pos(i, j, n);
+            sg[q] = pair_energy(p, a, g[i], g[j]);
+            mob[q] = pair_mobility(p, a, g[i], g[j]);
+        }
     {
         // the forward's arithmetic in R (list_compute_kernel / warp_general_kernel / list_step)
         const R norm_1r = (R)(1.0 / localN);
         const R prefr = (R)p.pref_do;
-        for (int i = 0; i < n; i++)
+        if (plain)
         {
-            const double vri = a.vr[g[i]];
-            const R vi = (R)val[i], li = (R)lap[i];
-            for (int j = i + 1; j < n; j++)
-            {
-                const int q = pair_pos(i, j, n);
-                const double vrj = a.vr[g[j]];
-                const R scale = (vri == 1.0 && vrj == 1.0) ? R(1) : (R)sqrt(vri * vrj);
-                const R h = R(0.5) * (R(1) + scale) * prefr;
-                const R vj = (R)val[j];
-                R dphi = (R)pair_energy(p, a, g[i], g[j]) * ((li + h * vi) - ((R)lap[j] + h * vj));
-                if (n > 2)
+            R sum[KL];
+            for (int k = 0; k < n; k++) sum[k] = (R)lap[k] + prefr * (R)val[k];
+            for (int i = 0; i < n; i++)
+                for (int j = i + 1; j < n; j++)
                 {
+                    const int q = pair_pos(i, j, n);
+                    R dphi = (R)sg[q] * (sum[i] - sum[j]);
                     for (int k = 0; k < n; k++)
                     {
                         if (k == i || k == j) continue;
-                        const R sbk = (R)pair_energy(p, a, g[j], g[k]);
-                        const R sak = (R)pair_energy(p, a, g[i], g[k]);
-                        const R vk = (R)val[k];
-                        dphi += (sbk - sak) * ((R)lap[k] + h * vk);
-                        if (p.tj_factor != 0.0 || scale < R(1))
+                        const R sbk = (R)sg[j < k ? pair_pos(j, k, n) : pair_pos(k, j, n)];
+                        const R sak = (R)sg[i < k ? pair_pos(i, k, n) : pair_pos(k, i, n)];
+                        dphi += (sbk - sak) * sum[k];
+                    }
+                    psi[q] = (double)dphi;
+                    dphi *= (R)mob[q] * norm_1r;
+                    pv0[q] = (double)dphi;
+                }
+        }
+        else
+        {
+            for (int i = 0; i < n; i++)
+            {
+                const R vi = (R)val[i], li = (R)lap[i];
+                for (int j = i + 1; j < n; j++)
+                {
+                    const int q = pair_pos(i, j, n);
+                    const R scale = (vr[i] == 1.0 && vr[j] == 1.0) ? R(1) : (R)sqrt(vr[i] * vr[j]);
+                    const R h = R(0.5) * (R(1) + scale) * prefr;
+                    const R vj = (R)val[j];
+                    R dphi = (R)sg[q] * ((li + h * vi) - ((R)lap[j] + h * vj));
+                    if (n > 2)
+                    {
+                        for (int k = 0; k < n; k++)
                         {
-                            const int pA = a.gphase[g[i]], pB = a.gphase[g[j]], pG = a.gphase[g[k]];
-                            const int P = p.nphases;
-                            const R tj = (R)dmax_ref(p.tj_factor, (double)(R(1) - scale));
-                            dphi += tj * prefr
-                                  * (((R)p.sigma_p[pA * P + pB] + (R)p.sigma_p[pB * P + pG]) + (R)p.sigma_p[pA * P + pG])
-                                  * (vi * vk - vj * vk);
+                            if (k == i || k == j) continue;
+                            const R sbk = (R)sg[j < k ? pair_pos(j, k, n) : pair_pos(k, j, n)];
+                            const R sak = (R)sg[i < k ? pair_pos(i, k, n) : pair_pos(k, i, n)];
+                            const R vk = (R)val[k];
+                            dphi += (sbk - sak) * ((R)lap[k] + h * vk);
+                            if (p.tj_factor != 0.0 || scale < R(1))
+                            {
+                                const int pA = a.gphase[g[i]], pB = a.gphase[g[j]], pG = a.gphase[g[k]];
+                                const int P = p.nphases;
+                                const R tj = (R)dmax_ref(p.tj_factor, (double)(R(1) - scale));
+                                dphi += tj * prefr
+                                      * (((R)p.sigma_p[pA * P + pB] + (R)p.sigma_p[pB * P + pG]) + (R)p.sigma_p[pA * P + pG])
+                                      * (vi * vk - vj * vk);
+                            }
                         }
                     }
+                    psi[q] = (double)dphi;
+                    dphi *= (R)mob[q] * norm_1r * scale;
+                    pv0[q] = (double)dphi;
                 }
-                psi[q] = (double)dphi;
-                dphi *= (R)pair_mobility(p, a, g[i], g[j]) * norm_1r * scale;
-                pv0[q] = (double)dphi;
             }
         }
     }
@@ -605,12 +648,14 @@ __device__ __forceinline__ void adjoint_core(const StepParams& p, const StepArra
                 const double locdG = limited_force(p, a, g[i], g[j]);
                 double norm = sqrt(val[i] * val[j]);
                 if (a.gstage[g[i]] == 1 || a.gstage[g[j]] == 1) norm += 1.0e-6;
-                pv0[pair_pos(i, j, n)] += locdG * (double)(R)pair_mobility(p, a, g[i], g[j]) * norm * p.pref_df;
+                pv0[pair_pos(i, j, n)] += locdG * (double)(R)mob[pair_pos(i, j, n)] * norm * p.pref_df;
             }
     }
     // ---- forward recompute: projection ----
     uint32_t zeroed = 0;       // fields whose increments the bound check zeroed
-    int iters = 0;             // limiter iterations run
+    int iters = 0;             // limiter iterations that acted (one where no field leaves [0, 1] is the
+                               // identity and has nothing to reverse)
+    bool any = false;          // the limiter ran
     bool single_clip = false;  // one pair: the increment was scaled onto the bound
     bool single_zero = false;
     double pos[KL], neg[KL], limN[KL], limP[KL], lpos[KL], lneg[KL];
@@ -651,19 +696,20 @@ __device__ __forceinline__ void adjoint_core(const StepParams& p, const StepArra
                     if (j != i) pv[i < j ? pair_pos(i, j, n) : pair_pos(j, i, n)] = 0.0;
             }
         }
-        bool any = false;
         for (int q = 0; q < np; q++) any |= (pv[q] != 0.0);
         if (any)
         {
             for (int it = 1; it <= 25; it++)
             {
+                const int acted = limiter_iteration(n, val, dt, pv, pos, neg, limN, limP);
+                if (acted == 0) break;
                 iters = it;
-                if (!limiter_iteration(n, val, dt, pv, pos, neg, limN, limP)) break;
+                if (acted == 1) break;
             }
         }
     }
     uint64_t epsmask0 = 0, epsmask1 = 0;   // pairs dropped by |pv*dt| < DBL_EPSILON (after the limiter)
-    if (np > 1 && iters > 0)
+    if (any)
         for (int q = 0; q < np; q++)
             if (fabs(pv[q] * dt) < DBL_EPSILON)
             {
@@ -778,78 +824,93 @@ __device__ __forceinline__ void adjoint_core(const StepParams& p, const StepArra
                 for (int j = 0; j < n; j++)
                     if (j != i) lpv[i < j ? pair_pos(i, j, n) : pair_pos(j, i, n)] = 0.0;
     }
-    // ---- reverse: driving force ----
-    if (with_dg)
-    {
-        for (int i = 0; i < n; i++)
-            for (int j = i + 1; j < n; j++)
-            {
-                const int q = pair_pos(i, j, n);
-                if (lpv[q] == 0.0) continue;
-                const double F = limited_force(p, a, g[i], g[j]);
-                const double mob = pair_mobility(p, a, g[i], g[j]);
-                const double s = sqrt(val[i] * val[j]);
-                double norm = s;
-                if (a.gstage[g[i]] == 1 || a.gstage[g[j]] == 1) norm += 1.0e-6;
-                const long long key = pair_key(g[i], g[j], G);
-                atomicAdd(&aa.gmu[key], lpv[q] * F * norm * p.pref_df);
-                const double lF = lpv[q] * mob * norm * p.pref_df;
-                const double dFb = lF * force_slope(p, a, g[i], g[j], F);
-                atomicAdd(&aa.gdg[g[j]], dFb);
-                atomicAdd(&aa.gdg[g[i]], -dFb);
-                if (s > 0.0)
-                {
-                    const double ln = lpv[q] * F * mob * p.pref_df;
-                    lval[i] += ln * val[j] / (2.0 * s);
-                    lval[j] += ln * val[i] / (2.0 * s);
-                }
-            }
-    }
-    // ---- reverse: pair kinetics ----
+    // ---- reverse: driving force and pair kinetics ----
+    // The parameter gradients of the voxel are summed per pair and field first: one global atomic per
+    // pair and parameter.
+    double gd[KL], lP[KL], gs[KP];
+    for (int k = 0; k < n; k++) { gd[k] = 0.0; lP[k] = 0.0; }
+    for (int q = 0; q < np; q++) gs[q] = 0.0;
     for (int i = 0; i < n; i++)
     {
-        const double vri = a.vr[g[i]];
         for (int j = i + 1; j < n; j++)
         {
             const int q = pair_pos(i, j, n);
             if (lpv[q] == 0.0) continue;
-            const double vrj = a.vr[g[j]];
-            const double scale = (vri == 1.0 && vrj == 1.0) ? 1.0 : sqrt(vri * vrj);
-            const double h = 0.5 * (1.0 + scale) * pref;
-            const double mob = pair_mobility(p, a, g[i], g[j]);
-            const long long key = pair_key(g[i], g[j], G);
-            atomicAdd(&aa.gmu[key], lpv[q] * psi[q] * norm_1 * scale);
-            const double lpsi = lpv[q] * mob * norm_1 * scale;
-            const double sij = pair_energy(p, a, g[i], g[j]);
-            atomicAdd(&aa.gsig[key], lpsi * ((lap[i] + h * val[i]) - (lap[j] + h * val[j])));
-            llap[i] += lpsi * sij; lval[i] += lpsi * sij * h;
-            llap[j] -= lpsi * sij; lval[j] -= lpsi * sij * h;
-            if (n > 2)
+            const double scale = (vr[i] == 1.0 && vr[j] == 1.0) ? 1.0 : sqrt(vr[i] * vr[j]);
+            double dmu = psi[q] * norm_1 * scale;
+            if (with_dg)
             {
-                for (int k = 0; k < n; k++)
+                const double F = limited_force(p, a, g[i], g[j]);
+                const double s = sqrt(val[i] * val[j]);
+                double norm = s;
+                if (a.gstage[g[i]] == 1 || a.gstage[g[j]] == 1) norm += 1.0e-6;
+                dmu += F * norm * p.pref_df;
+                const double lF = lpv[q] * mob[q] * norm * p.pref_df;
+                const double dFb = lF * force_slope(p, a, g[i], g[j], F);
+                gd[j] += dFb;
+                gd[i] -= dFb;
+                if (s > 0.0)
                 {
-                    if (k == i || k == j) continue;
-                    const double sbk = pair_energy(p, a, g[j], g[k]);
-                    const double sak = pair_energy(p, a, g[i], g[k]);
-                    const double Sk = lap[k] + h * val[k];
-                    atomicAdd(&aa.gsig[pair_key(g[j], g[k], G)], lpsi * Sk);
-                    atomicAdd(&aa.gsig[pair_key(g[i], g[k], G)], -lpsi * Sk);
-                    llap[k] += lpsi * (sbk - sak);
-                    lval[k] += lpsi * (sbk - sak) * h;
-                    if (p.tj_factor != 0.0 || scale < 1.0)
-                    {
-                        const int pA = a.gphase[g[i]], pB = a.gphase[g[j]], pG = a.gphase[g[k]];
-                        const int P = p.nphases;
-                        const double tj = dmax_ref(p.tj_factor, 1.0 - scale);
-                        const double ck = tj * pref * ((p.sigma_p[pA * P + pB] + p.sigma_p[pB * P + pG]) + p.sigma_p[pA * P + pG]);
-                        lval[i] += lpsi * ck * val[k];
-                        lval[j] -= lpsi * ck * val[k];
-                        lval[k] += lpsi * ck * (val[i] - val[j]);
-                    }
+                    const double ln = lpv[q] * F * mob[q] * p.pref_df;
+                    lval[i] += ln * val[j] / (2.0 * s);
+                    lval[j] += ln * val[i] / (2.0 * s);
+                }
+            }
+            atomicAdd(&aa.gmu[pair_key(g[i], g[j], G)], lpv[q] * dmu);
+            const double lpsi = lpv[q] * mob[q] * norm_1 * scale;
+            if (plain)
+            {
+                lP[j] += lpsi;
+                lP[i] -= lpsi;
+                continue;
+            }
+            const double h = 0.5 * (1.0 + scale) * pref;
+            gs[q] += lpsi * ((lap[i] + h * val[i]) - (lap[j] + h * val[j]));
+            llap[i] += lpsi * sg[q]; lval[i] += lpsi * sg[q] * h;
+            llap[j] -= lpsi * sg[q]; lval[j] -= lpsi * sg[q] * h;
+            for (int k = 0; k < n; k++)
+            {
+                if (k == i || k == j) continue;
+                const int qb = j < k ? pair_pos(j, k, n) : pair_pos(k, j, n);
+                const int qa = i < k ? pair_pos(i, k, n) : pair_pos(k, i, n);
+                const double Sk = lap[k] + h * val[k];
+                gs[qb] += lpsi * Sk;
+                gs[qa] -= lpsi * Sk;
+                llap[k] += lpsi * (sg[qb] - sg[qa]);
+                lval[k] += lpsi * (sg[qb] - sg[qa]) * h;
+                if (p.tj_factor != 0.0 || scale < 1.0)
+                {
+                    const int pA = a.gphase[g[i]], pB = a.gphase[g[j]], pG = a.gphase[g[k]];
+                    const int P = p.nphases;
+                    const double tj = dmax_ref(p.tj_factor, 1.0 - scale);
+                    const double ck = tj * pref * ((p.sigma_p[pA * P + pB] + p.sigma_p[pB * P + pG]) + p.sigma_p[pA * P + pG]);
+                    lval[i] += lpsi * ck * val[k];
+                    lval[j] -= lpsi * ck * val[k];
+                    lval[k] += lpsi * ck * (val[i] - val[j]);
                 }
             }
         }
     }
+    if (plain)
+    {
+        // With S = lap + pref*val and P_i = sum_k sigma_ik S_k every increment is P_j - P_i (the terms of
+        // the pair itself and of the third fields together), so the reverse of all pairs goes through
+        // the n adjoints of P: pairs instead of pairs times third fields.
+        for (int i = 0; i < n; i++)
+            for (int j = i + 1; j < n; j++)
+            {
+                const int q = pair_pos(i, j, n);
+                gs[q] = lP[i] * (lap[j] + pref * val[j]) + lP[j] * (lap[i] + pref * val[i]);
+                llap[i] += sg[q] * lP[j];
+                llap[j] += sg[q] * lP[i];
+            }
+        for (int k = 0; k < n; k++) lval[k] += pref * llap[k];
+    }
+    for (int i = 0; i < n; i++)
+        for (int j = i + 1; j < n; j++)
+            if (gs[pair_pos(i, j, n)] != 0.0) atomicAdd(&aa.gsig[pair_key(g[i], g[j], G)], gs[pair_pos(i, j, n)]);
+    for (int k = 0; k < n; k++)
+        if (gd[k] != 0.0) atomicAdd(&aa.gdg[g[k]], gd[k]);
     // ---- outputs ----
     for (int s = 0; s < c; s++) aa.lam_local[s * N + v] = lval[s];
     aa.lcnt[v] = (uint8_t)n;
