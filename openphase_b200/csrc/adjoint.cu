@@ -12,7 +12,7 @@
 // the step reads them: table, hash or phase pair) and the per-grain driving force dG(g).
 //
 // Kernels
-//   tlm_step_kernel      one forward step of the FP64 form with dual numbers: new state + tangent
+//   tlm_*_kernel         one forward step of the FP64 form with dual numbers: new state + tangent
 //   adjoint_core         per wide voxel: recompute the step's arithmetic (same operation order as
 //                        the forward), reverse it: adjoint of the voxel's own input values, of the
 //                        Laplacians of its list, and the parameter gradients; driven by
@@ -86,7 +86,7 @@ __device__ __forceinline__ double force_slope(const StepParams& p, const StepArr
 // Stages 2-5 of list_step<double> on dual numbers, operation by operation in the same order, so the
 // value parts are the forward's bit for bit and every decision is the forward's.
 template <int KL>
-__device__ int stages_dual(const StepParams& p, const StepArrays& a, const AdjArrays& aa, int n, int flag,
+__device__ __forceinline__ int stages_dual(const StepParams& p, const StepArrays& a, const AdjArrays& aa, int n, int flag,
                            int16_t* g, Dual* val, const Dual* lap, Dual* sg, Dual* pv, Dual* pos, Dual* neg,
                            uint32_t& st)
 {
@@ -106,37 +106,61 @@ __device__ int stages_dual(const StepParams& p, const StepArrays& a, const AdjAr
         for (int j = i + 1; j < n; j++)
             sg[pair_pos(i, j, n)] = mkd(pair_energy(p, a, g[i], g[j]), aa.tsig ? aa.tsig[pair_key(g[i], g[j], G)] : 0.0);
     const double pref = p.pref_do;
-    for (int i = 0; i < n; i++)
+    bool plain = p.tj_factor == 0.0;   // as in list_compute_kernel: one sum per field
+    for (int k = 0; k < n; k++) plain = plain && a.vr[g[k]] == 1.0;
+    if (plain)
     {
-        const double vri = a.vr[g[i]];
-        for (int j = i + 1; j < n; j++)
-        {
-            const int q = pair_pos(i, j, n);
-            const double vrj = a.vr[g[j]];
-            const double scale = (vri == 1.0 && vrj == 1.0) ? 1.0 : sqrt(vri * vrj);
-            const double h = 0.5 * (1.0 + scale) * pref;
-            Dual dphi = sg[q] * ((lap[i] + h * val[i]) - (lap[j] + h * val[j]));
-            if (n > 2)
+        for (int k = 0; k < n; k++) pos[k] = lap[k] + pref * val[k];
+        for (int i = 0; i < n; i++)
+            for (int j = i + 1; j < n; j++)
             {
+                const int q = pair_pos(i, j, n);
+                Dual dphi = sg[q] * (pos[i] - pos[j]);
                 for (int k = 0; k < n; k++)
                 {
                     if (k == i || k == j) continue;
                     const Dual sbk = sg[j < k ? pair_pos(j, k, n) : pair_pos(k, j, n)];
                     const Dual sak = sg[i < k ? pair_pos(i, k, n) : pair_pos(k, i, n)];
-                    dphi = dphi + (sbk - sak) * (lap[k] + h * val[k]);
-                    if (p.tj_factor != 0.0 || scale < 1.0)
+                    dphi = dphi + (sbk - sak) * pos[k];
+                }
+                const Dual mob = mkd(pair_mobility(p, a, g[i], g[j]), aa.tmu ? aa.tmu[pair_key(g[i], g[j], G)] : 0.0);
+                pv[q] = dphi * (mob * norm_1);
+            }
+    }
+    else
+    {
+        for (int i = 0; i < n; i++)
+        {
+            const double vri = a.vr[g[i]];
+            for (int j = i + 1; j < n; j++)
+            {
+                const int q = pair_pos(i, j, n);
+                const double vrj = a.vr[g[j]];
+                const double scale = (vri == 1.0 && vrj == 1.0) ? 1.0 : sqrt(vri * vrj);
+                const double h = 0.5 * (1.0 + scale) * pref;
+                Dual dphi = sg[q] * ((lap[i] + h * val[i]) - (lap[j] + h * val[j]));
+                if (n > 2)
+                {
+                    for (int k = 0; k < n; k++)
                     {
-                        const int pA = a.gphase[g[i]], pB = a.gphase[g[j]], pG = a.gphase[g[k]];
-                        const int P = p.nphases;
-                        const double tj = dmax_ref(p.tj_factor, 1.0 - scale);
-                        dphi = dphi + tj * pref * ((p.sigma_p[pA * P + pB] + p.sigma_p[pB * P + pG]) + p.sigma_p[pA * P + pG])
-                                    * (val[i] * val[k] - val[j] * val[k]);
+                        if (k == i || k == j) continue;
+                        const Dual sbk = sg[j < k ? pair_pos(j, k, n) : pair_pos(k, j, n)];
+                        const Dual sak = sg[i < k ? pair_pos(i, k, n) : pair_pos(k, i, n)];
+                        dphi = dphi + (sbk - sak) * (lap[k] + h * val[k]);
+                        if (p.tj_factor != 0.0 || scale < 1.0)
+                        {
+                            const int pA = a.gphase[g[i]], pB = a.gphase[g[j]], pG = a.gphase[g[k]];
+                            const int P = p.nphases;
+                            const double tj = dmax_ref(p.tj_factor, 1.0 - scale);
+                            dphi = dphi + tj * pref * ((p.sigma_p[pA * P + pB] + p.sigma_p[pB * P + pG]) + p.sigma_p[pA * P + pG])
+                                        * (val[i] * val[k] - val[j] * val[k]);
+                        }
                     }
                 }
+                const Dual mob = mkd(pair_mobility(p, a, g[i], g[j]), aa.tmu ? aa.tmu[pair_key(g[i], g[j], G)] : 0.0);
+                dphi = dphi * ((mob * norm_1) * scale);
+                pv[q] = dphi;
             }
-            const Dual mob = mkd(pair_mobility(p, a, g[i], g[j]), aa.tmu ? aa.tmu[pair_key(g[i], g[j], G)] : 0.0);
-            dphi = dphi * ((mob * norm_1) * scale);
-            pv[q] = dphi;
         }
     }
     if (p.use_dg && flag == 2)
@@ -203,16 +227,19 @@ __device__ int stages_dual(const StepParams& p, const StepArrays& a, const AdjAr
                         if (w.v < 0.0) { neg[i] = neg[i] + w; pos[j] = pos[j] + (-w); }
                         if (w.v > 0.0) { pos[i] = pos[i] + w; neg[j] = neg[j] + (-w); }
                     }
+                bool outside = false;
                 for (int i = 0; i < n; i++)
                 {
                     const Dual vi = val[i], pi = pos[i], ni = neg[i];
                     const Dual newPF = vi + (pi + ni) * dt;
+                    outside = outside || newPF.v < 0.0 || newPF.v > 1.0;
                     Dual limN = mkd(1.0), limP = mkd(1.0);
                     if (newPF.v < 0.0) limN = dmin_d(mkd(1.0), -(vi + pi * dt) / (ni * dt));
                     if (newPF.v > 1.0) limP = dmin_d(mkd(1.0), (1.0 - (vi + ni * dt)) / (pi * dt));
                     neg[i] = limN;
                     pos[i] = limP;
                 }
+                if (!outside) break;   // every limit is 1
                 bool needed = false;
                 for (int i = 0; i < n; i++)
                     for (int j = i + 1; j < n; j++)
@@ -294,84 +321,175 @@ __device__ __forceinline__ int find_entry(const uint8_t* cnt, const int16_t* idx
     return -1;
 }
 
-template <int KS, int KL>
-__global__ void __launch_bounds__(128) tlm_step_kernel(const __grid_constant__ StepParams p, const StepArrays a,
-                                                        const AdjArrays aa)
+// The tangent step runs on the forward's lists: the classify kernel leaves the list, values and
+// Laplacians of every wide voxel of up to kListCap fields (and copies the bulk voxels), and here
+//   tlm_list_kernel      adds the tangents (the list's own and their Laplacians, from the neighbours in
+//                        global memory) and runs the stages on dual numbers, one thread per voxel,
+//                        a kernel per list length beside each other;
+//   tlm_worklist_kernel  does the same for the general-path worklist with the general gather;
+//   tlm_bulk_kernel      carries the bulk voxels' tangents over.
+// Bound: latency of the neighbour loads and of the stages' arrays; the lists sort the voxels by length,
+// so that a warp's lanes run the same loops over arrays of their own length.
+struct TlmBlock {
+    int key[kTileVolSlots];
+    double sum[kTileVolSlots], tan[kTileVolSlots];
+    unsigned long long cnt[3];
+};
+
+__device__ __forceinline__ void tlm_block_begin(TlmBlock& B)
 {
-    __shared__ int s_key[kVolSlots];
-    __shared__ double s_sum[kVolSlots];
-    __shared__ unsigned long long s_cnt[3];
-    for (int i = threadIdx.x; i < kVolSlots; i += blockDim.x) { s_key[i] = -1; s_sum[i] = 0.0; }
-    if (threadIdx.x < 3) s_cnt[threadIdx.x] = 0ull;
+    for (int i = threadIdx.x; i < kTileVolSlots; i += blockDim.x) { B.key[i] = -1; B.sum[i] = 0.0; B.tan[i] = 0.0; }
+    if (threadIdx.x < 3) B.cnt[threadIdx.x] = 0ull;
     __syncthreads();
-    const long long N = p.n;
-    const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t st = 0;
-    unsigned wide = 0, ein = 0, eout = 0;
-    if (v < N)
+}
+
+// Volume and volume tangent of one stored field.
+__device__ __forceinline__ void tlm_volume(TlmBlock& B, const StepArrays& a, const AdjArrays& aa, int g, double v, double d)
+{
+    unsigned h = ((unsigned)g * 2654435761u) & (unsigned)(kTileVolSlots - 1);
+    for (int probe = 0; probe < kTileVolSlots; probe++)
     {
-        const uint8_t* cnt = a.cnt_in;
-        const int16_t* gin = a.idx_in;
-        const double* vin = static_cast<const double*>(a.val_in);
-        double* vout = static_cast<double*>(a.val_out);
-        const Neighbourhood nb(p, v);
-        const int c = cnt[v];
-        ein = c;
-        const int flag = voxel_flag(cnt, nb, v);
-        if (flag == 0)
+        const int k = atomicCAS(&B.key[h], -1, g);
+        if (k == -1 || k == g)
         {
-            a.cnt_out[v] = (uint8_t)c;
-            for (int s = 0; s < c; s++)
-            {
-                const int g = gin[s * N + v];
-                a.idx_out[s * N + v] = (int16_t)g;
-                vout[s * N + v] = vin[s * N + v];
-                aa.dphi_out[s * N + v] = aa.dphi_in[s * N + v];
-                vol_insert_n(s_key, s_sum, kVolSlots, a.vol_acc, g, vin[s * N + v]);
-                atomicAdd(&aa.tvol[g], aa.dphi_in[s * N + v]);
-            }
-            eout = c;
+            if (v != 0.0) atomicAdd(&B.sum[h], v);
+            atomicAdd(&B.tan[h], d);
+            return;
         }
-        else
+        h = (h + 1) & (unsigned)(kTileVolSlots - 1);
+    }
+    atomicAdd(&a.vol_acc[g], v);
+    atomicAdd(&aa.tvol[g], d);
+}
+
+__device__ __forceinline__ void tlm_block_end(TlmBlock& B, const StepArrays& a, const AdjArrays& aa, unsigned eout, uint32_t st)
+{
+    flush_block(a, 0u, 0u, eout, st, B.cnt, B.key, B.sum, kTileVolSlots, threadIdx.x, blockDim.x);
+    for (int i = threadIdx.x; i < kTileVolSlots; i += blockDim.x)
+        if (B.key[i] >= 0) atomicAdd(&aa.tvol[B.key[i]], B.tan[i]);
+}
+
+// One wide voxel from its list: tangents, stages, new record.
+template <int KS, int KL>
+__device__ __forceinline__ int tlm_voxel(const StepParams& p, const StepArrays& a, const AdjArrays& aa, TlmBlock& B,
+                                         long long v, int flag, int n, int c, int16_t* g, const double* vr,
+                                         const double* lr, uint32_t& st)
+{
+    constexpr int KP = KL * (KL - 1) / 2;
+    const long long N = p.n;
+    double* vout = static_cast<double*>(a.val_out);
+    Dual val[KL], lap[KL], sg[KP], pv[KP], pos[KL], neg[KL];
+    for (int k = 0; k < n; k++)
+    {
+        val[k] = mkd(vr[k], k < c ? aa.dphi_in[k * N + v] : 0.0);
+        lap[k] = mkd(lr[k], 0.0);
+    }
+    // tangent of the Laplacians: the same stencil over the neighbours' tangents
+    const Neighbourhood nb(p, v);
+    for (int q = 0; q < p.ns; q++)
+    {
+        const long long u = nb_at(nb, p.lap_d[q]);
+        const int cu = a.cnt_in[u];
+        for (int s = 0; s < cu; s++)
         {
-            wide = 1;
-            constexpr int KP = KL * (KL - 1) / 2;
-            int16_t gL[KL];
-            double vr[KL], lr[KL];
-            const int n = gather_list<double, KL>(p, cnt, gin, vin, nb, v, gL, vr, lr, nullptr, st);
-            Dual val[KL], lap[KL], sg[KP], pv[KP], pos[KL], neg[KL];
+            const int gu = a.idx_in[s * N + u];
+            const double d = aa.dphi_in[s * N + u];
             for (int k = 0; k < n; k++)
-            {
-                val[k] = mkd(vr[k], k < c ? aa.dphi_in[k * N + v] : 0.0);
-                lap[k] = mkd(lr[k], 0.0);
-            }
-            // tangent of the Laplacians: the same stencil over the neighbours' tangents
-            for (int q = 0; q < p.ns; q++)
-            {
-                const long long u = nb.at(p.lap_d[q][0], p.lap_d[q][1], p.lap_d[q][2]);
-                const int cu = cnt[u];
-                for (int s = 0; s < cu; s++)
-                {
-                    const int g = gin[s * N + u];
-                    for (int k = 0; k < n; k++)
-                        if (gL[k] == g) { lap[k].d += p.lap_w[q] * aa.dphi_in[s * N + u]; break; }
-                }
-            }
-            int m = stages_dual<KL>(p, a, aa, n, flag, gL, val, lap, sg, pv, pos, neg, st);
-            if (m > KS) { st |= kStOverflowK; m = KS; }
-            a.cnt_out[v] = (uint8_t)m;
-            for (int i = 0; i < m; i++)
-            {
-                a.idx_out[i * N + v] = gL[i];
-                vout[i * N + v] = val[i].v;
-                aa.dphi_out[i * N + v] = val[i].d;
-                vol_insert_n(s_key, s_sum, kVolSlots, a.vol_acc, gL[i], val[i].v);
-                atomicAdd(&aa.tvol[gL[i]], val[i].d);
-            }
-            eout = m;
+                if (g[k] == gu) { lap[k].d += p.lap_w[q] * d; break; }
         }
     }
-    flush_block(a, wide, ein, eout, st, s_cnt, s_key, s_sum, kVolSlots, threadIdx.x, blockDim.x);
+    int m = stages_dual<KL>(p, a, aa, n, flag, g, val, lap, sg, pv, pos, neg, st);
+    if (m > KS) { st |= kStOverflowK; m = KS; }
+    a.cnt_out[v] = (uint8_t)m;
+    for (int i = 0; i < m; i++)
+    {
+        a.idx_out[i * N + v] = g[i];
+        vout[i * N + v] = val[i].v;
+        aa.dphi_out[i * N + v] = val[i].d;
+        tlm_volume(B, a, aa, g[i], val[i].v, val[i].d);
+    }
+    return m;
+}
+
+template <int N>
+__global__ void __launch_bounds__(128) tlm_list_kernel(const __grid_constant__ StepParams p, const StepArrays a,
+                                                        const AdjArrays aa, int nslices)
+{
+    __shared__ TlmBlock B;
+    const unsigned* __restrict__ off = a.bucket_off + (long long)N * (nslices + 1);
+    const unsigned total = off[nslices];
+    const unsigned per = ((total + gridDim.x * blockDim.x - 1u) / (gridDim.x * blockDim.x)) * blockDim.x;
+    const unsigned r0 = blockIdx.x * per;
+    if (r0 >= total) return;
+    const unsigned r1 = min(total, r0 + per);
+    tlm_block_begin(B);
+    const int2* __restrict__ buck = a.bucket + (long long)N * a.bucket_cap;
+    constexpr int kPad = ((2 * N + 7) / 8) * 8;
+    uint32_t st = 0;
+    unsigned eout = 0;
+    for (unsigned e = r0 + threadIdx.x; e < r1; e += blockDim.x)
+    {
+        const int sl = slice_of(off, nslices, e);
+        const int2 ent = buck[(long long)sl * a.slice + (e - off[sl])];
+        const unsigned char* __restrict__ w = a.wl + (long long)sl * a.wl_slice + ent.y;
+        const long long v = ent.x & 0x7fffffff;
+        int16_t g[N];
+#pragma unroll
+        for (int k = 0; k < N; k++) g[k] = reinterpret_cast<const int16_t*>(w)[k];
+        const double* vr = reinterpret_cast<const double*>(w + kPad);
+        eout += tlm_voxel<kListCap, N>(p, a, aa, B, v, (ent.x >> 31) ? 2 : 1, N, (int)a.cnt_in[v], g, vr, vr + N, st);
+    }
+    tlm_block_end(B, a, aa, eout, st);
+}
+
+template <int KS>
+__global__ void __launch_bounds__(64) tlm_worklist_kernel(const __grid_constant__ StepParams p, const StepArrays a,
+                                                           const AdjArrays aa)
+{
+    __shared__ TlmBlock B;
+    tlm_block_begin(B);
+    const unsigned total = min(*a.slow_count, a.slow_cap);
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&a.counters[kCntGeneralLast], (unsigned long long)total);
+    const unsigned warps = gridDim.x * (blockDim.x >> 5);
+    const unsigned warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    uint32_t st = 0;
+    unsigned eout = 0;
+    for (unsigned i = (threadIdx.x & 31u) * warps + warp; i < total; i += 32u * warps)   // as the adjoint's worklist
+    {
+        const long long v = a.slow_list[i];
+        const Neighbourhood nb(p, v);
+        int16_t g[KAdjList];
+        double vr[KAdjList], lr[KAdjList];
+        const int n = gather_list<double, KAdjList>(p, a.cnt_in, a.idx_in, static_cast<const double*>(a.val_in), nb, v, g,
+                                                    vr, lr, nullptr, st);
+        eout += tlm_voxel<KS, KAdjList>(p, a, aa, B, v, voxel_flag(a.cnt_in, nb, v), n, (int)a.cnt_in[v], g, vr, lr, st);
+    }
+    tlm_block_end(B, a, aa, eout, st);
+}
+
+// Bulk voxels: the tangent is carried over (the classify kernel has copied the state and its volumes).
+__global__ void __launch_bounds__(128) tlm_bulk_kernel(const __grid_constant__ StepParams p, const StepArrays a,
+                                                        const AdjArrays aa)
+{
+    __shared__ TlmBlock B;
+    tlm_block_begin(B);
+    const long long N = p.n;
+    const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (v < N)
+    {
+        const Neighbourhood nb(p, v);
+        if (voxel_flag(a.cnt_in, nb, v) == 0)
+        {
+            const int c = a.cnt_in[v];
+            for (int s = 0; s < c; s++)
+            {
+                const double d = aa.dphi_in[s * N + v];
+                aa.dphi_out[s * N + v] = d;
+                tlm_volume(B, a, aa, a.idx_in[s * N + v], 0.0, d);
+            }
+        }
+    }
+    tlm_block_end(B, a, aa, 0u, 0u);
 }
 
 // ---- adjoint -------------------------------------------------------------------------------------
@@ -987,8 +1105,12 @@ __global__ void __launch_bounds__(64) adjoint_worklist_kernel(const __grid_const
                                                                const AdjArrays aa)
 {
     constexpr int KL = KAdjList;
+    // Each voxel is one long chain with branches of its own: consecutive voxels go to different warps,
+    // so that a warp holds as few of them as there are warps for.
     const unsigned total = min(*a.slow_count, a.slow_cap);
-    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x)
+    const unsigned warps = gridDim.x * (blockDim.x >> 5);
+    const unsigned warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    for (unsigned i = (threadIdx.x & 31u) * warps + warp; i < total; i += 32u * warps)
     {
         const long long v = a.slow_list[i];
         const Neighbourhood nb(p, v);
@@ -1157,16 +1279,29 @@ __global__ void lambda_init_kernel(long long N, const uint8_t* __restrict__ cnt,
 
 static unsigned grid_of(long long n, int t) { return (unsigned)((n + t - 1) / t); }
 
-int launch_tlm_step(const StepParams& p, const StepArrays& a, const AdjArrays& aa, int k_slots, void* stream)
+int launch_tlm_step(const StepParams& p, const StepArrays& a, const AdjArrays& aa, int k_slots, int nblocks, void* stream,
+                    const SideStreams& side)
 {
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const SideFork fork(&side, static_cast<cudaStream_t>(stream));
+    bool known = true;
     switch (k_slots)
     {
-        case 8:  tlm_step_kernel<8, KAdjList><<<grid_of(p.n, 128), 128, 0, s>>>(p, a, aa); break;
-        case 12: tlm_step_kernel<12, KAdjList><<<grid_of(p.n, 128), 128, 0, s>>>(p, a, aa); break;
-        case 16: tlm_step_kernel<16, KAdjList><<<grid_of(p.n, 128), 128, 0, s>>>(p, a, aa); break;
-        default: return -1;
+        case 8:  tlm_worklist_kernel<8><<<148 * 8, 64, 0, fork.on(0)>>>(p, a, aa); break;
+        case 12: tlm_worklist_kernel<12><<<148 * 8, 64, 0, fork.on(0)>>>(p, a, aa); break;
+        case 16: tlm_worklist_kernel<16><<<148 * 8, 64, 0, fork.on(0)>>>(p, a, aa); break;
+        default: known = false; break;
     }
+    tlm_list_kernel<8><<<148 * 8, 128, 0, fork.on(1)>>>(p, a, aa, nblocks);
+    tlm_list_kernel<7><<<148 * 8, 128, 0, fork.on(2)>>>(p, a, aa, nblocks);
+    tlm_list_kernel<6><<<148 * 8, 128, 0, fork.main>>>(p, a, aa, nblocks);
+    tlm_list_kernel<5><<<148 * 8, 128, 0, fork.on(3)>>>(p, a, aa, nblocks);
+    tlm_list_kernel<4><<<148 * 8, 128, 0, fork.main>>>(p, a, aa, nblocks);
+    tlm_list_kernel<3><<<148 * 8, 128, 0, fork.on(3)>>>(p, a, aa, nblocks);
+    tlm_list_kernel<2><<<148 * 8, 128, 0, fork.on(2)>>>(p, a, aa, nblocks);
+    tlm_bulk_kernel<<<grid_of(p.n, 128), 128, 0, fork.main>>>(p, a, aa);
+    const cudaError_t e = fork.join();
+    if (!known) return -1;
+    if (e != cudaSuccess) return (int)e;
     return (int)cudaGetLastError();
 }
 
@@ -1181,7 +1316,7 @@ static void adjoint_kernels(const StepParams& p, const StepArrays& a, const AdjA
                             const SideFork& fork)
 {
     const cudaStream_t s = fork.main;
-    adjoint_worklist_kernel<R, KS><<<148 * 4, 64, 0, fork.on(2)>>>(p, a, aa);
+    adjoint_worklist_kernel<R, KS><<<148 * 8, 64, 0, fork.on(2)>>>(p, a, aa);
     adjoint_list_kernel<R, 8><<<kAdjListBlocks, 128, 0, fork.on(0)>>>(p, a, aa, nblocks);
     adjoint_list_kernel<R, 7><<<kAdjListBlocks, 128, 0, fork.on(1)>>>(p, a, aa, nblocks);
     adjoint_list_kernel<R, 6><<<kAdjListBlocks, 128, 0, s>>>(p, a, aa, nblocks);

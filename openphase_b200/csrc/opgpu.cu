@@ -1765,6 +1765,7 @@ extern "C" uint32_t opgpu_tlm_step(opgpu_ctx* ctx, double dt, int32_t nsteps)
     if (uint32_t r = refresh_dg_pair(ctx)) return r;
     StepParams sp = ctx->sp;
     sp.dt = dt;
+    sp.vol_x0 = 0; sp.vol_x1 = sp.nx;   // the tangent model sums the volumes of the whole grid
     for (int s = 0; s < nsteps; s++)
     {
         const int in = ctx->cur, out = 1 - ctx->cur;
@@ -1774,12 +1775,15 @@ extern "C" uint32_t opgpu_tlm_step(opgpu_ctx* ctx, double dt, int32_t nsteps)
         aa.dphi_in = ctx->d_dphi[ctx->dphi_cur]; aa.dphi_out = ctx->d_dphi[1 - ctx->dphi_cur];
         aa.tvol = ctx->d_tvol;
         CK(cudaMemsetAsync(ctx->d_tvol, 0, (size_t)ctx->G * sizeof(double), ctx->stream));
-        CK(cudaMemsetAsync(aa.dphi_out, 0, (size_t)ctx->n * ctx->K * sizeof(double), ctx->stream));
-        if (launch_tlm_step(sp, a, aa, ctx->K, ctx->stream)) return fail(ctx, OPGPU_E_CUDA, "opgpu_tlm_step: launch");
+        set_worklists(ctx, a);
+        const int nblocks = launch_classify_f64(sp, a, ctx->stream);
+        if (nblocks < 0) return fail(ctx, OPGPU_E_CUDA, "opgpu_tlm_step: classify launch");
+        // every stored entry of the new state gets its tangent
+        if (launch_tlm_step(sp, a, aa, ctx->K, nblocks, ctx->stream, ctx->side)) return fail(ctx, OPGPU_E_CUDA, "opgpu_tlm_step: launch");
         grains_update_kernel<<<grid_for(ctx->G, 256), 256, 0, ctx->stream>>>(ctx->G, ctx->d_vol_acc, ctx->d_volume,
             ctx->d_maxvol, ctx->d_refvol, ctx->d_vr, ctx->d_exist, ctx->d_gstage, ctx->d_counters, 1);
         CK(cudaGetLastError());
-        ctx->kernel_launches += 2;
+        ctx->kernel_launches += 12;
         ctx->cur = out;
         ctx->dphi_cur = 1 - ctx->dphi_cur;
     }
