@@ -140,6 +140,26 @@ void dfree(void* p)
 
 __device__ __forceinline__ double dmax_ref(double a, double b) { return (a < b) ? b : a; }
 
+// Per-block grain-volume table of the list upload: neighbouring voxels share few grains, one global
+// atomic per stored field serialised on the grains' addresses (128^3, 250 grains: 615 us).
+constexpr int kLoadVolSlots = 256;
+
+__device__ __forceinline__ void load_volume(int* keys, double* sums, double* vol_acc, int g, double v)
+{
+    unsigned h = ((unsigned)g * 2654435761u) & (unsigned)(kLoadVolSlots - 1);
+    for (int probe = 0; probe < kLoadVolSlots; probe++)
+    {
+        const int k = atomicCAS(&keys[h], -1, g);
+        if (k == -1 || k == g)
+        {
+            atomicAdd(&sums[h], v);
+            return;
+        }
+        h = (h + 1) & (unsigned)(kLoadVolSlots - 1);
+    }
+    atomicAdd(&vol_acc[g], v);
+}
+
 // Ragged lists -> K-slot state; voxels with more than one entry go through NodePF::finalize
 // (include/Containers/NodePF.h:214-255), which FinalizeSR applies to the flag-2 voxels that
 // NodePF::read produced (NodePF.h:751-763).
@@ -149,9 +169,12 @@ __global__ void load_kernel(long long N, int K, int G, const int32_t* counts, co
                             R* val_out, uint32_t* status, double* vol_acc)
 {
     const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= N) return;
-    const int c = counts[v];
-    const long long off = offsets[v];
+    __shared__ int s_key[kLoadVolSlots];
+    __shared__ double s_sum[kLoadVolSlots];
+    for (int i = threadIdx.x; i < kLoadVolSlots; i += blockDim.x) { s_key[i] = -1; s_sum[i] = 0.0; }
+    __syncthreads();
+    const int c = v < N ? counts[v] : 0;
+    const long long off = v < N ? offsets[v] : 0;
     uint32_t st = 0;
     if (c > 1)
     {
@@ -187,10 +210,10 @@ __global__ void load_kernel(long long N, int K, int G, const int32_t* counts, co
         {
             idx_out[i * N + v] = (int16_t)gs[i];
             val_out[i * N + v] = (R)vs[i];
-            atomicAdd(&vol_acc[gs[i]], (double)(R)vs[i]);
+            load_volume(s_key, s_sum, vol_acc, gs[i], (double)(R)vs[i]);
         }
     }
-    else
+    else if (v < N)
     {
         if (c == 0) st |= kStEmptyVoxel;
         cnt_out[v] = (uint8_t)c;
@@ -198,10 +221,13 @@ __global__ void load_kernel(long long N, int K, int G, const int32_t* counts, co
         {
             idx_out[v] = (int16_t)idx[off];
             val_out[v] = (R)val[off];
-            atomicAdd(&vol_acc[idx[off]], (double)(R)val[off]);
+            load_volume(s_key, s_sum, vol_acc, idx[off], (double)(R)val[off]);
         }
     }
     if (st) atomicOr(status, st);
+    __syncthreads();
+    for (int i = threadIdx.x; i < kLoadVolSlots; i += blockDim.x)
+        if (s_key[i] >= 0) atomicAdd(&vol_acc[s_key[i]], s_sum[i]);
 }
 
 // PhaseField::CalculateGrainsVolume tail (src/PhaseField.cpp:896-951): MAXVolume, VolumeRatio,
@@ -1501,8 +1527,8 @@ StepArrays step_arrays(opgpu_ctx* ctx, const uint8_t* cnt_in, const int16_t* idx
 }
 
 // Counts and stored fields of a state (slots beyond a voxel's count hold nothing).  Bound: bandwidth of
-// the slots in use; at 256^3, K = 16, FP64 the voxels hold two fields of sixteen, so copying whole slot
-// planes moved 5.4 GB.
+// the slots in use; at 256^3, K = 16, FP64 the voxels hold two fields of sixteen and copying whole slot
+// planes moved 5.4 GB (846 -> 426 us).
 template <class R>
 __global__ void __launch_bounds__(256) copy_fields_kernel(long long N, const uint8_t* __restrict__ sc,
                                                            const int16_t* __restrict__ si, const R* __restrict__ sv,
@@ -1868,7 +1894,7 @@ static uint32_t plane_copy(opgpu_ctx* ctx, int32_t x, void* buf, bool pack)
     if (P % 16 == 0 && reinterpret_cast<uintptr_t>(buf) % 16 == 0 && at.type == cudaMemoryTypeDevice && at.device == ctx->device)
     {
         // every part starts on 16 bytes (N is a multiple of P): one kernel instead of three copies, two
-        // of them strided (256^3, K = 16, FP64: 17 -> 5 us a plane)
+        // of them strided (256^3, K = 16, FP64: 18 -> 8 us a plane)
         const unsigned vecs = (unsigned)(P / 16), rsz = (unsigned)ctx->rsz;
         const unsigned gx = std::min(64u, (rsz * vecs + 255u) / 256u);
         plane_copy_kernel<<<dim3(gx, 1u + 2u * (unsigned)K), 256, 0, ctx->stream>>>(
