@@ -73,6 +73,7 @@ struct opgpu_ctx {
     std::vector<double> h_dg_pair;      // [G*G] host side of the limited driving-force table
     bool pair_energy_dirty = true;
     uint32_t* d_status = nullptr;
+    unsigned char* h_stage = nullptr;   // pinned: the status word, then the grain records on their way out
     unsigned long long* d_counters = nullptr;
     int* d_slow_list = nullptr;      // overflow worklist of the tiled kernel (capacity N)
     unsigned* d_slow_count = nullptr;
@@ -111,6 +112,7 @@ struct opgpu_ctx {
 namespace {
 
 constexpr double kPi = 3.14159265358979323846;   // include/Globals.h:124
+constexpr size_t kStageHead = 64;                // bytes of the pinned staging before the grain records
 
 uint32_t fail(opgpu_ctx* c, uint32_t code, const std::string& msg)
 {
@@ -496,10 +498,11 @@ void set_stencils(StepParams& sp, int lap, int grad, double dx)
 
 uint32_t read_status(opgpu_ctx* ctx)
 {
-    uint32_t st = 0;
-    CK(cudaMemcpyAsync(&st, ctx->d_status, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
+    uint32_t* word = reinterpret_cast<uint32_t*>(ctx->h_stage);
+    CK(cudaMemcpyAsync(word, ctx->d_status, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaMemsetAsync(ctx->d_status, 0, sizeof(uint32_t), ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
+    const uint32_t st = *word;
     for (size_t i = 0; i < ctx->ev_used; i++)
     {
         float ms = 0.f, ms_c = 0.f;
@@ -609,6 +612,7 @@ extern "C" uint32_t opgpu_create(const opgpu_grid* grid, opgpu_ctx** out)
             return bail(OPGPU_E_CUDA);
     }
     if (dalloc(&ctx->d_status, 1) != cudaSuccess) return bail(OPGPU_E_CUDA);
+    if (cudaMallocHost(reinterpret_cast<void**>(&ctx->h_stage), kStageHead) != cudaSuccess) return bail(OPGPU_E_CUDA);
     if (dalloc(&ctx->d_counters, kNumCounters) != cudaSuccess) return bail(OPGPU_E_CUDA);
     cudaMemset(ctx->d_status, 0, sizeof(uint32_t));
     cudaMemset(ctx->d_counters, 0, kNumCounters * sizeof(unsigned long long));
@@ -644,6 +648,7 @@ extern "C" uint32_t opgpu_destroy(opgpu_ctx* ctx)
     dfree(ctx->d_facets);
     dfree(ctx->d_avg_strong); dfree(ctx->d_avg_mask); dfree(ctx->d_avg_off);
     dfree(ctx->d_status);
+    if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
     dfree(ctx->d_counters);
     for (auto& s : ctx->slots)
     {
@@ -815,6 +820,12 @@ extern "C" uint32_t opgpu_set_grains(opgpu_ctx* ctx, int32_t ngrains, const int3
         gs[g] = (int8_t)s;
     }
     free_grains(ctx);
+    {
+        unsigned char* stage = nullptr;
+        CK(cudaMallocHost(reinterpret_cast<void**>(&stage), kStageHead + (size_t)G * (3 * sizeof(double) + 2)));
+        cudaFreeHost(ctx->h_stage);
+        ctx->h_stage = stage;
+    }
     ctx->G = G;
     ctx->sp.ngrains = G;
     CK(dalloc(&ctx->d_vr, G));
@@ -1432,24 +1443,26 @@ extern "C" uint32_t opgpu_grains(opgpu_ctx* ctx, double* volume, double* volume_
                                  int32_t* exist, int32_t* stage)
 {
     if (uint32_t r = require(ctx, ctx && ctx->G > 0, "no grains")) return r;
-    const int G = ctx->G;
+    // the records asked for go through pinned memory behind the steps enqueued so far: one wait for all
+    const size_t G = (size_t)ctx->G;
+    double* h = reinterpret_cast<double*>(ctx->h_stage + kStageHead);
+    int8_t* h8 = reinterpret_cast<int8_t*>(h + 3 * G);
+    auto fetch = [&](void* to, const void* from, size_t bytes) {
+        return cudaMemcpyAsync(to, from, bytes, cudaMemcpyDeviceToHost, ctx->stream);
+    };
+    if (volume) CK(fetch(h, ctx->d_volume, G * sizeof(double)));
+    if (volume_ratio) CK(fetch(h + G, ctx->d_vr, G * sizeof(double)));
+    if (max_volume) CK(fetch(h + 2 * G, ctx->d_maxvol, G * sizeof(double)));
+    if (exist) CK(fetch(h8, ctx->d_exist, G));
+    if (stage) CK(fetch(h8 + G, ctx->d_gstage, G));
     CK(cudaStreamSynchronize(ctx->stream));
-    if (volume) CK(cudaMemcpy(volume, ctx->d_volume, G * sizeof(double), cudaMemcpyDeviceToHost));
-    if (volume_ratio) CK(cudaMemcpy(volume_ratio, ctx->d_vr, G * sizeof(double), cudaMemcpyDeviceToHost));
-    if (max_volume) CK(cudaMemcpy(max_volume, ctx->d_maxvol, G * sizeof(double), cudaMemcpyDeviceToHost));
-    if (exist || stage)
+    if (volume) std::memcpy(volume, h, G * sizeof(double));
+    if (volume_ratio) std::memcpy(volume_ratio, h + G, G * sizeof(double));
+    if (max_volume) std::memcpy(max_volume, h + 2 * G, G * sizeof(double));
+    for (size_t g = 0; g < G; g++)
     {
-        std::vector<int8_t> tmp(G);
-        if (exist)
-        {
-            CK(cudaMemcpy(tmp.data(), ctx->d_exist, G, cudaMemcpyDeviceToHost));
-            for (int g = 0; g < G; g++) exist[g] = tmp[g];
-        }
-        if (stage)
-        {
-            CK(cudaMemcpy(tmp.data(), ctx->d_gstage, G, cudaMemcpyDeviceToHost));
-            for (int g = 0; g < G; g++) stage[g] = tmp[g];
-        }
+        if (exist) exist[g] = h8[g];
+        if (stage) stage[g] = h8[G + g];
     }
     return OPGPU_OK;
 }
