@@ -37,7 +37,13 @@ struct WindowSlots {
 };
 constexpr int kSlotMap = 512;        // grain -> slot map entries
 constexpr int kTileVolSlots = 512;      // grain-volume hash of the compute kernels
-constexpr int kKeepEntries = 6;         // entries per record the plane loader keeps in registers
+// Entries per record the plane loader keeps in registers.  FP32 has 96 registers at five blocks per SM
+// and spills with six (256^3, classify: 1894 us with six, 1760 with four); FP64 has 160 at three blocks,
+// and the records beyond four cost more (2060 with six, 2178 with four).
+template <class R>
+struct KeepEntries {
+    static constexpr int value = sizeof(R) == 8 ? 6 : 4;
+};
 constexpr int kClassifyVolSlots = 128;  // grain-volume hash of the classify kernel (bulk voxels)
 // Blocks of each per-length compute kernel: one per 4096 voxels of the grid, between 8 and 32 per
 // SM (a finer split of each length's entries pays on large grids; on small ones the per-block
@@ -132,12 +138,10 @@ __device__ __forceinline__ int find_slot(const S& sm, int g)
     return sm.grain_of[k] == g ? k : search_slot(sm, g);
 }
 
-// Records of a ring plane each thread handles, and how many entries of each it keeps in registers
-// between the two passes of load_plane.
+// Records of a ring plane each thread handles.
 template <int TY>
 struct PlaneRegs {
     static constexpr int kPer = (TileGeom<TY>::kRecs + TileGeom<TY>::NT - 1) / TileGeom<TY>::NT;
-    static constexpr int kKeep = kKeepEntries;
 };
 
 // In-plane offset of record r (the same in every plane; -1 beyond the last record).
@@ -179,13 +183,13 @@ __device__ __forceinline__ void plane_begin(const StepParams& p, const StepArray
     prefetch_counts<TY>(p, a, xp, P);
 }
 
-// Registers a thread keeps between the passes of the plane loader: the first kKeep entries of each
+// Registers a thread keeps between the passes of the plane loader: the first KeepEntries entries of each
 // of its records, the slots found so far (4 bits an entry, entries 0-7 and 8-15) and the entries
 // without one.
 template <class R, int TY>
 struct PlaneLoad {
-    int gr[PlaneRegs<TY>::kPer][PlaneRegs<TY>::kKeep];
-    R vr[PlaneRegs<TY>::kPer][PlaneRegs<TY>::kKeep];
+    int gr[PlaneRegs<TY>::kPer][KeepEntries<R>::value];
+    R vr[PlaneRegs<TY>::kPer][KeepEntries<R>::value];
     uint32_t lst[PlaneRegs<TY>::kPer][2];
     uint32_t miss[PlaneRegs<TY>::kPer];
 };
@@ -197,15 +201,15 @@ __device__ __forceinline__ int kept_grain(const PlaneLoad<R, TY>& L, int i, int 
 {
     int g = 0;
 #pragma unroll
-    for (int q = 0; q < PlaneRegs<TY>::kKeep; q++)
+    for (int q = 0; q < KeepEntries<R>::value; q++)
         if (q == s) g = L.gr[i][q];
-    return s >= PlaneRegs<TY>::kKeep ? (int)gin[s * N] : g;
+    return s >= KeepEntries<R>::value ? (int)gin[s * N] : g;
 }
 
 // Bringing plane xp (window position wpos) into ring slot `rs` -- slot lists, bitmask words and
 // dense per-slot values; grains not yet in the window get a slot that no grain of the window uses --
 // takes three passes with a barrier between each:
-//   plane_scan    reads the records once (the first kKeep entries stay in registers) and finds their
+//   plane_scan    reads the records once (the first KeepEntries entries stay in registers) and finds their
 //                 slots through the map; marks the slots as in use and collects the grains without
 //                 one in `pending`; it touches only map and grain_of (read), lastpos and pending, so
 //                 it may run while other threads still read the ring for the previous plane; returns
@@ -229,7 +233,7 @@ __device__ __forceinline__ bool plane_scan(const StepParams& p, const StepArrays
 #pragma unroll
     for (int i = 0; i < PR::kPer; i++)
 #pragma unroll
-        for (int s = 0; s < PR::kKeep; s++)
+        for (int s = 0; s < KeepEntries<R>::value; s++)
             if (s < P.cr[i])
             {
                 L.gr[i][s] = gin[s * N + P.off[i]];
@@ -240,9 +244,9 @@ __device__ __forceinline__ bool plane_scan(const StepParams& p, const StepArrays
     {
         const int c = P.cr[i];
         uint32_t lst[2] = {0u, 0u};
-        uint32_t miss = c > PR::kKeep ? ((1u << c) - 1u) & ~((1u << PR::kKeep) - 1u) : 0u;
+        uint32_t miss = c > KeepEntries<R>::value ? ((1u << c) - 1u) & ~((1u << KeepEntries<R>::value) - 1u) : 0u;
 #pragma unroll
-        for (int s = 0; s < PR::kKeep; s++)
+        for (int s = 0; s < KeepEntries<R>::value; s++)
             if (s < c)
             {
                 const int g = L.gr[i][s], k = S.map[slot_hash(g)];
@@ -339,14 +343,14 @@ __device__ __forceinline__ void plane_fill(const StepParams& p, const StepArrays
         }
         uint32_t msk = 0;
 #pragma unroll
-        for (int s = 0; s < PR::kKeep; s++)
+        for (int s = 0; s < KeepEntries<R>::value; s++)
             if (s < c && !((lost >> s) & 1u))
             {
                 const int k = (int)(lst[0] >> (4 * s)) & 15;
                 S.dense[k].at[rs][r] = L.vr[i][s];
                 msk |= 1u << k;
             }
-        for (int s = PR::kKeep; s < c; s++)
+        for (int s = KeepEntries<R>::value; s < c; s++)
             if (!((lost >> s) & 1u))
             {
                 const int k = (int)(lst[s >> 3] >> (4 * (s & 7))) & 15;
@@ -667,7 +671,8 @@ static __global__ void __launch_bounds__(1024) bucket_scan_kernel(const StepArra
 }
 
 constexpr int kChunkTable = 128;   // 32-entry chunks of a compute block whose slices are tabulated
-constexpr int kVolCache = 4;       // per-thread grain-volume cache of the compute kernels
+constexpr int kVolCache = 2;       // per-thread grain-volume cache of the compute kernels (four entries, of
+                                   // which a thread's few voxels fill most once: FP32 step 4072 -> 4002 us)
 
 // Stages 2-5 for lists of exactly N fields (compile-time), all arrays in registers; the operation
 // order is that of list_step.  The entries of length N from all classify slices form one index
@@ -682,8 +687,10 @@ constexpr int kVolCache = 4;       // per-thread grain-volume cache of the compu
 //
 // N <= kListCap <= the stored fields per voxel, so a new record always fits.  AVG: averaged driving
 // forces (a template parameter: the mask costs the plain step registers).
+// Resident blocks: six for N <= 3, five for 4 and 5, three beyond (the registers each takes unbounded
+// allow five, four and two to three): FP64 step at 256^3 4365 -> 4298 us.
 template <class R, int N, bool AVG>
-__global__ void __launch_bounds__(128) list_compute_kernel(const __grid_constant__ StepParams p, const StepArrays a,
+__global__ void __launch_bounds__(128, N <= 3 ? 6 : (N <= 5 ? 5 : 3)) list_compute_kernel(const __grid_constant__ StepParams p, const StepArrays a,
                                                            int nslices)
 {
     constexpr int NP = N * (N - 1) / 2;
