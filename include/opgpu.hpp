@@ -231,7 +231,7 @@ public:
         Phi.check(opgpu_set_averaging(Phi.ctx_, Averaging ? 1 : 0, Range, Threshold), "DrivingForce::ReadInput");
     }
     /* DrivingForce::Average (src/DrivingForce.cpp:242-256): with averaging on, SetWeights,
-     * CollectAverage and DistributeAverage run inside the fused step on the state it starts from;
+     * CollectAverage and DistributeAverage run (as one reach test) on the state the step starts from;
      * else SkipAverage (:258-274). */
     void Average(PhaseField&, const BoundaryConditions&) {}
     void MergePhaseFieldIncrements(PhaseField& Phi, InterfaceProperties&)
