@@ -680,10 +680,11 @@ constexpr int kVolCache = 2;       // per-thread grain-volume cache of the compu
 // consecutive entries at a time, so that no warp idles while another drains a long slice.
 //
 // Bound: issue and latency at 16-20 warps per SM -- FP64 arithmetic, pair-table loads and, for long
-// lists, instruction fetch -- not bandwidth (N = 4 at 256^3: 0.45 ms for 0.09 ms of traffic).  Leaving
+// lists, instruction fetch -- not bandwidth (N = 4 at 256^3: 0.41 ms for 0.09 ms of traffic).  Leaving
 // out what repeats (one sum per field instead of one per pair and third field, one pass for merge and
 // plausibility, no limits where no field leaves [0, 1]) took N = 2..8 at 256^3, FP64, from 235 443 519
-// 396 283 185 147 us to 235 391 452 305 219 131 129.
+// 396 283 185 147 us to 235 391 452 305 219 131 129 (233 389 412 281 206 126 117 with the block bounds and the
+// smaller volume cache below).
 //
 // N <= kListCap <= the stored fields per voxel, so a new record always fits.  AVG: averaged driving
 // forces (a template parameter: the mask costs the plain step registers).
