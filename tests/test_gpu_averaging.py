@@ -2,10 +2,10 @@
 
 The oracle's restatement of DrivingForce::Average is pinned to the reference by the fixtures
 tests/golden/average_*.npz (tests/test_oracle.py); here the CUDA path (opgpu_set_averaging) is held
-to the oracle and to those fixtures.  The averaged force of each voxel pair goes through CUDA's tanh
-in the limiter (the value differs per voxel, so no per-pair table applies), which can differ from
-the C library's in the last bit: the bar is the parity bar (identical lists, borderline voxels
-counted, max|dphi| <= 1e-9) over the tested windows.
+to the oracle and to those fixtures.  The device decides per pair and voxel whether the averaged force
+is the raw force or none, and takes the pair's tabulated force; the reference's quotient of sums
+differs from it by rounding: the bar is the parity bar (identical lists, borderline voxels counted,
+max|dphi| <= 1e-9) over the tested windows.
 """
 from pathlib import Path
 
