@@ -284,7 +284,9 @@ void*    opgpu_stream(opgpu_ctx* ctx);
  * gradient accumulation are FP64.  The tangent-linear model runs the FP64 form. */
 /* Reserve nslots device checkpoints (state plus grain records). */
 uint32_t opgpu_checkpoint_reserve(opgpu_ctx* ctx, int32_t nslots);
-/* Copy the current state and grain records into / out of a checkpoint slot. */
+/* Copy the current state and grain records into / out of a checkpoint slot.  A slot that was reserved
+ * but never saved (by opgpu_checkpoint_save or opgpu_step_save_input) holds no state: loading it or
+ * stepping back to it (opgpu_adjoint_step) is refused with OPGPU_E_STATE. */
 uint32_t opgpu_checkpoint_save(opgpu_ctx* ctx, int32_t slot);
 uint32_t opgpu_checkpoint_load(opgpu_ctx* ctx, int32_t slot);
 /* One step (opgpu_step with nsteps = 1) that leaves the state it started from, with its grain

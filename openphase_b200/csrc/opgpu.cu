@@ -50,6 +50,7 @@ struct opgpu_ctx {
         uint8_t* cnt = nullptr; int16_t* idx = nullptr; void* val = nullptr;
         double *volume = nullptr, *maxvol = nullptr, *vr = nullptr;
         int8_t *exist = nullptr, *stage = nullptr;
+        bool saved = false;              // holds a state (a reserved slot's memory is not cleared)
     };
     std::vector<Slot> slots;
     // adjoint / tangent-linear buffers (allocated on first use)
@@ -1539,18 +1540,18 @@ StepArrays step_arrays(opgpu_ctx* ctx, const uint8_t* cnt_in, const int16_t* idx
     return a;
 }
 
-// Counts and stored fields of a state (slots beyond a voxel's count hold nothing).  Bound: bandwidth of
-// the slots in use; at 256^3, K = 16, FP64 the voxels hold two fields of sixteen and copying whole slot
-// planes moved 5.4 GB (846 -> 426 us).
+// Counts and stored fields of a state (slots beyond a voxel's count hold nothing; no count takes the
+// copy past the K planes of its buffers).  Bound: bandwidth of the slots in use; at 256^3, K = 16, FP64
+// the voxels hold two fields of sixteen and copying whole slot planes moved 5.4 GB (846 -> 426 us).
 template <class R>
-__global__ void __launch_bounds__(256) copy_fields_kernel(long long N, const uint8_t* __restrict__ sc,
+__global__ void __launch_bounds__(256) copy_fields_kernel(long long N, int K, const uint8_t* __restrict__ sc,
                                                            const int16_t* __restrict__ si, const R* __restrict__ sv,
                                                            uint8_t* __restrict__ dc, int16_t* __restrict__ di,
                                                            R* __restrict__ dv)
 {
     const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= N) return;
-    const int c = sc[v];
+    const int c = min((int)sc[v], K);
     dc[v] = (uint8_t)c;
     for (int s = 0; s < c; s++)
     {
@@ -1563,11 +1564,11 @@ uint32_t copy_state(opgpu_ctx* ctx, uint8_t* dc, int16_t* di, void* dv, const ui
                     const void* sv)
 {
     if (ctx->fp32)
-        copy_fields_kernel<<<grid_for(ctx->n, 256), 256, 0, ctx->stream>>>(ctx->n, sc, si, static_cast<const float*>(sv),
-                                                                          dc, di, static_cast<float*>(dv));
+        copy_fields_kernel<<<grid_for(ctx->n, 256), 256, 0, ctx->stream>>>(
+            ctx->n, ctx->K, sc, si, static_cast<const float*>(sv), dc, di, static_cast<float*>(dv));
     else
-        copy_fields_kernel<<<grid_for(ctx->n, 256), 256, 0, ctx->stream>>>(ctx->n, sc, si, static_cast<const double*>(sv),
-                                                                          dc, di, static_cast<double*>(dv));
+        copy_fields_kernel<<<grid_for(ctx->n, 256), 256, 0, ctx->stream>>>(
+            ctx->n, ctx->K, sc, si, static_cast<const double*>(sv), dc, di, static_cast<double*>(dv));
     CK(cudaGetLastError());
     return OPGPU_OK;
 }
@@ -1662,9 +1663,12 @@ extern "C" uint32_t opgpu_checkpoint_save(opgpu_ctx* ctx, int32_t slot)
     if (uint32_t r = require(ctx, ctx && ctx->initialized, "opgpu_checkpoint_save: not initialized")) return r;
     if (slot < 0 || slot >= (int)ctx->slots.size()) return fail(ctx, OPGPU_E_INVALID, "opgpu_checkpoint_save: no such slot");
     auto& s = ctx->slots[slot];
+    s.saved = false;
     if (uint32_t r = copy_state(ctx, s.cnt, s.idx, s.val, ctx->cnt[ctx->cur], ctx->idx[ctx->cur], ctx->val[ctx->cur])) return r;
-    return copy_grains(ctx, s.volume, s.maxvol, s.vr, s.exist, s.stage, ctx->d_volume, ctx->d_maxvol, ctx->d_vr,
-                       ctx->d_exist, ctx->d_gstage);
+    if (uint32_t r = copy_grains(ctx, s.volume, s.maxvol, s.vr, s.exist, s.stage, ctx->d_volume, ctx->d_maxvol, ctx->d_vr,
+                                 ctx->d_exist, ctx->d_gstage)) return r;
+    s.saved = true;
+    return OPGPU_OK;
 }
 
 extern "C" uint32_t opgpu_step_save_input(opgpu_ctx* ctx, double dt, int32_t slot)
@@ -1673,6 +1677,7 @@ extern "C" uint32_t opgpu_step_save_input(opgpu_ctx* ctx, double dt, int32_t slo
     if (slot < 0 || slot >= (int)ctx->slots.size()) return fail(ctx, OPGPU_E_INVALID, "opgpu_step_save_input: no such slot");
     auto& s = ctx->slots[slot];
     // the grain records are updated in place by the step: copy them first (G values)
+    s.saved = false;
     if (uint32_t r = copy_grains(ctx, s.volume, s.maxvol, s.vr, s.exist, s.stage, ctx->d_volume, ctx->d_maxvol,
                                  ctx->d_vr, ctx->d_exist, ctx->d_gstage)) return r;
     const int in = ctx->cur;
@@ -1682,6 +1687,7 @@ extern "C" uint32_t opgpu_step_save_input(opgpu_ctx* ctx, double dt, int32_t slo
     std::swap(ctx->cnt[in], s.cnt);
     std::swap(ctx->idx[in], s.idx);
     std::swap(ctx->val[in], s.val);
+    s.saved = true;
     return opgpu_sync(ctx);
 }
 
@@ -1690,6 +1696,7 @@ extern "C" uint32_t opgpu_checkpoint_load(opgpu_ctx* ctx, int32_t slot)
     if (uint32_t r = require(ctx, ctx && ctx->initialized, "opgpu_checkpoint_load: not initialized")) return r;
     if (slot < 0 || slot >= (int)ctx->slots.size()) return fail(ctx, OPGPU_E_INVALID, "opgpu_checkpoint_load: no such slot");
     auto& s = ctx->slots[slot];
+    if (!s.saved) return fail(ctx, OPGPU_E_STATE, "opgpu_checkpoint_load: nothing was saved in this slot");
     if (uint32_t r = copy_state(ctx, ctx->cnt[ctx->cur], ctx->idx[ctx->cur], ctx->val[ctx->cur], s.cnt, s.idx, s.val)) return r;
     if (uint32_t r = copy_grains(ctx, ctx->d_volume, ctx->d_maxvol, ctx->d_vr, ctx->d_exist, ctx->d_gstage,
                                  s.volume, s.maxvol, s.vr, s.exist, s.stage)) return r;
@@ -1723,8 +1730,9 @@ extern "C" uint32_t opgpu_adjoint_step(opgpu_ctx* ctx, int32_t slot, double dt)
     if (uint32_t r = require(ctx, ctx && ctx->adjoint_ready, "opgpu_adjoint_step: call opgpu_adjoint_begin first")) return r;
     if (slot < 0 || slot >= (int)ctx->slots.size()) return fail(ctx, OPGPU_E_INVALID, "opgpu_adjoint_step: no such slot");
     if (!(dt > 0.0)) return fail(ctx, OPGPU_E_INVALID, "opgpu_adjoint_step: dt > 0 required");
-    if (uint32_t r = refresh_dg_pair(ctx)) return r;
     auto& s = ctx->slots[slot];
+    if (!s.saved) return fail(ctx, OPGPU_E_STATE, "opgpu_adjoint_step: nothing was saved in this slot");
+    if (uint32_t r = refresh_dg_pair(ctx)) return r;
     StepParams sp = ctx->sp;
     sp.dt = dt;
     StepArrays a = step_arrays(ctx, s.cnt, s.idx, s.val, s.vr, 1 - ctx->cur);

@@ -4,6 +4,8 @@ checkpoints restore a state exactly."""
 import numpy as np
 import pytest
 
+from openphase_b200._lib import E_STATE, OpgpuError
+from openphase_b200.adjoint import Rollout
 from openphase_b200.cases import Case
 from openphase_b200.context import Context
 
@@ -64,3 +66,32 @@ def test_checkpoint_restores_the_stored_fields(precision):
     ctx.checkpoint_load(0)
     for a, b in zip(ctx.download(), before):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_slots_that_were_never_saved_are_refused(precision):
+    """A reserved slot's memory holds whatever the device memory held before: its counts are not to be
+    trusted.  Loading it and stepping back to it are refused, and the state stays as it was."""
+    case, ctx = _ctx(17, 13, precision, 8)
+    w = np.ones(case.ngrains)
+    ctx.checkpoint_reserve(3)
+    ctx.checkpoint_save(0)
+    before = ctx.download()
+    ctx.adjoint_begin(w)
+    for call in (lambda: ctx.checkpoint_load(1), lambda: ctx.adjoint_step(2, case.dt)):
+        with pytest.raises(OpgpuError) as e:
+            call()
+        assert e.value.code & E_STATE
+    for a, b in zip(ctx.download(), before):
+        assert np.array_equal(a, b)
+    ctx.step_save_input(case.dt, 1)   # the ways to fill a slot
+    ctx.checkpoint_load(1)
+    for a, b in zip(ctx.download(), before):
+        assert np.array_equal(a, b)
+    R = Rollout(ctx, case.dt, 5)      # its segment slots are new
+    with pytest.raises(OpgpuError) as e:
+        R.backward(w)
+    assert e.value.code & E_STATE
+    R.forward()
+    R.backward(w)
+    assert R.adjoint_status == 0
