@@ -137,7 +137,8 @@ typedef struct opgpu_stats {
     int64_t general_path_total;    /* voxels processed by the general per-voxel path (long lists,
                                       windows with too many grains) summed over all steps          */
     int64_t crowded_window_total;  /* of those, voxels whose 3-plane window held too many grains  */
-    double  timed_classify_ms;     /* of timed_kernel_ms, the part spent in the classify kernel     */
+    double  timed_classify_ms;     /* of timed_kernel_ms, the part spent in the classify kernel, with
+                                      every model (the generic kernel variant has no such part)      */
     int64_t kernel_launches;       /* kernels this library launched for steps since creation       */
 } opgpu_stats;
 

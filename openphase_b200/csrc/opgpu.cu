@@ -1262,8 +1262,8 @@ static uint32_t enqueue_steps(opgpu_ctx* ctx, double dt, int nsteps, bool partia
                 }
             }
             CK(cudaEventRecord(ctx->ev_pool[3 * ctx->ev_used], ctx->stream));
-            // "after classify" is recorded at the start too; the tiled path records it again after
-            // its classify kernel (paths without a classify phase leave it at the start)
+            // "after classify" is recorded at the start too; the tiled step records it again after
+            // its classify kernel (the generic variant has none and leaves it at the start)
             CK(cudaEventRecord(ctx->ev_pool[3 * ctx->ev_used + 1], ctx->stream));
             info.after_classify = ctx->ev_pool[3 * ctx->ev_used + 1];
         }

@@ -1247,8 +1247,7 @@ int launch_tiled_ns(const StepParams& p, const StepArrays& a, void* stream, Laun
     e = cudaMemsetAsync(a.slow_count, 0, sizeof(unsigned), s);
     if (e != cudaSuccess) return (int)e;
     kern<<<dim3(gz, gy, gx), dim3(kTileZ, kTileTY), smem, s>>>(p, a, xchunk);
-    // (anisotropic steps report no classify share: their timing is that of the whole step)
-    if (info && info->after_classify && !p.aniso)
+    if (info && info->after_classify)
     {
         e = cudaEventRecord(static_cast<cudaEvent_t>(info->after_classify), s);
         if (e != cudaSuccess) return (int)e;
