@@ -8,6 +8,7 @@
 #include <cub/device/device_reduce.cuh>
 #include <cub/device/device_scan.cuh>
 #include <cuda_runtime.h>
+#include <sys/mman.h>
 
 #include <algorithm>
 #include <array>
@@ -75,6 +76,7 @@ struct opgpu_ctx {
     bool pair_energy_dirty = true;
     uint32_t* d_status = nullptr;
     unsigned char* h_stage = nullptr;   // pinned: the status word, then the grain records on their way out
+    size_t h_stage_bytes = 0;
     unsigned long long* d_counters = nullptr;
     int* d_slow_list = nullptr;      // overflow worklist of the tiled kernel (capacity N)
     unsigned* d_slow_count = nullptr;
@@ -140,6 +142,62 @@ void dfree(void* p)
 }
 
 // ------------------------------------------------------------------------------------ kernels
+
+// Pinned host memory of a context: registered pages.  While a process holds no other pinned block,
+// cudaMallocHost takes 0.8 to 2.7 ms and cudaFreeHost 0.4 ms; registering some pages takes 0.28 ms and
+// giving them back 0.17 ms.  (A child of fork() does not get the pages, so that the parent's stay where
+// the device writes them.)
+unsigned char* pinned_alloc(size_t bytes)
+{
+    void* p = mmap(nullptr, bytes, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+    if (p == MAP_FAILED) return nullptr;
+    madvise(p, bytes, MADV_DONTFORK);
+    if (cudaHostRegister(p, bytes, cudaHostRegisterDefault) == cudaSuccess) return static_cast<unsigned char*>(p);
+    cudaGetLastError();   // the caller reports it
+    munmap(p, bytes);
+    return nullptr;
+}
+
+void pinned_free(unsigned char* p, size_t bytes)
+{
+    if (!p) return;
+    cudaHostUnregister(p);
+    munmap(p, bytes);
+}
+
+// The staging block holds the status word and the records of G grains.  It is made with the grains (or
+// with a status word asked for before) and kept while it is large enough.
+constexpr size_t kStageFirst = 16384;   // some 600 grains
+bool reserve_stage(opgpu_ctx* ctx, int G)
+{
+    const size_t need = kStageHead + (size_t)G * (3 * sizeof(double) + 2);
+    if (need <= ctx->h_stage_bytes) return true;
+    const size_t bytes = std::max(kStageFirst, (need + 4095) / 4096 * 4096);
+    unsigned char* block = pinned_alloc(bytes);
+    if (!block) return false;
+    pinned_free(ctx->h_stage, ctx->h_stage_bytes);
+    ctx->h_stage = block;
+    ctx->h_stage_bytes = bytes;
+    return true;
+}
+
+// The context's side streams, made with the grains (some 0.24 ms: a context that never steps goes
+// without, and no step is the one that makes them).
+uint32_t make_side_streams(opgpu_ctx* ctx)
+{
+    SideStreams& s = ctx->side;
+    auto event = [](void** e) {
+        return *e ? cudaSuccess : cudaEventCreateWithFlags(reinterpret_cast<cudaEvent_t*>(e), cudaEventDisableTiming);
+    };
+    CK(event(&s.fork));
+    for (int k = 0; k < kSideStreams; k++)
+    {
+        if (!s.stream[k])
+            CK(cudaStreamCreateWithFlags(reinterpret_cast<cudaStream_t*>(&s.stream[k]), cudaStreamNonBlocking));
+        CK(event(&s.join[k]));
+    }
+    return OPGPU_OK;
+}
 
 __device__ __forceinline__ double dmax_ref(double a, double b) { return (a < b) ? b : a; }
 
@@ -499,6 +557,7 @@ void set_stencils(StepParams& sp, int lap, int grad, double dx)
 
 uint32_t read_status(opgpu_ctx* ctx)
 {
+    if (!reserve_stage(ctx, 0)) return fail(ctx, OPGPU_E_CUDA, "no pinned memory for the status word");
     uint32_t* word = reinterpret_cast<uint32_t*>(ctx->h_stage);
     CK(cudaMemcpyAsync(word, ctx->d_status, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaMemsetAsync(ctx->d_status, 0, sizeof(uint32_t), ctx->stream));
@@ -574,19 +633,6 @@ extern "C" uint32_t opgpu_create(const opgpu_grid* grid, opgpu_ctx** out)
     auto bail = [&](uint32_t code) { opgpu_destroy(ctx); return code; };
     if (cudaSetDevice(ctx->device) != cudaSuccess) return bail(OPGPU_E_CUDA);
     if (cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess) return bail(OPGPU_E_CUDA);
-    {
-        cudaEvent_t ev;
-        if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) return bail(OPGPU_E_CUDA);
-        ctx->side.fork = ev;
-        for (int k = 0; k < kSideStreams; k++)
-        {
-            cudaStream_t st;
-            if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) return bail(OPGPU_E_CUDA);
-            ctx->side.stream[k] = st;
-            if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) return bail(OPGPU_E_CUDA);
-            ctx->side.join[k] = ev;
-        }
-    }
     for (int b = 0; b < 2; b++)
     {
         if (dalloc(&ctx->cnt[b], (size_t)ctx->n) != cudaSuccess) return bail(OPGPU_E_CUDA);
@@ -613,7 +659,6 @@ extern "C" uint32_t opgpu_create(const opgpu_grid* grid, opgpu_ctx** out)
             return bail(OPGPU_E_CUDA);
     }
     if (dalloc(&ctx->d_status, 1) != cudaSuccess) return bail(OPGPU_E_CUDA);
-    if (cudaMallocHost(reinterpret_cast<void**>(&ctx->h_stage), kStageHead) != cudaSuccess) return bail(OPGPU_E_CUDA);
     if (dalloc(&ctx->d_counters, kNumCounters) != cudaSuccess) return bail(OPGPU_E_CUDA);
     cudaMemset(ctx->d_status, 0, sizeof(uint32_t));
     cudaMemset(ctx->d_counters, 0, kNumCounters * sizeof(unsigned long long));
@@ -649,7 +694,7 @@ extern "C" uint32_t opgpu_destroy(opgpu_ctx* ctx)
     dfree(ctx->d_facets);
     dfree(ctx->d_avg_strong); dfree(ctx->d_avg_mask); dfree(ctx->d_avg_off);
     dfree(ctx->d_status);
-    if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
+    pinned_free(ctx->h_stage, ctx->h_stage_bytes);
     dfree(ctx->d_counters);
     for (auto& s : ctx->slots)
     {
@@ -820,13 +865,9 @@ extern "C" uint32_t opgpu_set_grains(opgpu_ctx* ctx, int32_t ngrains, const int3
         if (s < 0 || s > 2) return fail(ctx, OPGPU_E_INVALID, "opgpu_set_grains: bad stage");
         gs[g] = (int8_t)s;
     }
+    if (!reserve_stage(ctx, G)) return fail(ctx, OPGPU_E_CUDA, "opgpu_set_grains: no pinned memory for the grain records");
+    if (uint32_t r = make_side_streams(ctx)) return r;
     free_grains(ctx);
-    {
-        unsigned char* stage = nullptr;
-        CK(cudaMallocHost(reinterpret_cast<void**>(&stage), kStageHead + (size_t)G * (3 * sizeof(double) + 2)));
-        cudaFreeHost(ctx->h_stage);
-        ctx->h_stage = stage;
-    }
     ctx->G = G;
     ctx->sp.ngrains = G;
     CK(dalloc(&ctx->d_vr, G));

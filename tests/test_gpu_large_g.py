@@ -53,3 +53,33 @@ def test_large_grain_count_matches_oracle(mode):
         live = go["volume"] > 0
         assert np.max(np.abs(g["volume"][live] - go["volume"][live]) / go["volume"][live]) <= 1e-12
         assert np.array_equal(g["exist"], go["exist"])
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_grain_records_follow_the_uploaded_lists(precision):
+    """Random lists of many grains: a block of the upload's 256 voxels holds more grains than its volume
+    table has places (the rest adds to the grains directly), and one context takes grain sets of growing
+    and shrinking size, so that the records outgrow their staging memory and fit it again."""
+    rng = np.random.default_rng(5)
+    n, ctx = 24 * 20 * 16, Context(24, 20, 16, precision=precision, k_slots=8)
+    ctx.set_model([[1.2]], [[1.0]])
+    for G in (12, 700, 5000, 5000, 30):
+        ctx.set_grains(G)
+        counts = rng.integers(1, 4, n).astype(np.int32)
+        first = np.repeat(rng.integers(0, G, n), counts)
+        place = np.arange(counts.sum()) - np.repeat(np.cumsum(counts) - counts, counts)
+        idx = ((first + place) % G).astype(np.int32)
+        val = rng.uniform(0.2, 0.8, idx.size)
+        val[np.repeat(counts == 1, counts)] = 1.0
+        if G == 5000:
+            starts = np.concatenate([[0], np.cumsum(counts)])[::256]
+            assert min(np.unique(idx[a:b]).size for a, b in zip(starts, starts[1:])) > 256
+        ctx.upload(counts, idx, val)
+        assert ctx.finalize_initialization() == 0
+        c, i, v = ctx.download()
+        assert np.array_equal(c, counts) and np.array_equal(i, idx)
+        expected = np.bincount(i, weights=v, minlength=G)
+        g = ctx.grains()
+        assert np.max(np.abs(g["volume"] - expected)) <= 1e-12 * n
+        assert np.array_equal(g["exist"], expected > 0)
+        assert np.array_equal(g["max_volume"], g["volume"]) and not g["stage"].any()
