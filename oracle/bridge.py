@@ -35,7 +35,8 @@ class OpParams(C.Structure):
                 ("mobility_facet_family", C.c_void_p), ("quat", C.c_void_p), ("pair_sigma", C.c_void_p), ("pair_mu", C.c_void_p), ("dg", C.c_void_p),
                 ("limiting", C.c_int), ("limit_phase", C.c_void_p), ("regularization", C.c_double),
                 ("tj_factor", C.c_double), ("consider_nucleus_volume", C.c_int),
-                ("nucleus_volume_factor", C.c_double), ("threads", C.c_int), ("average", C.c_int)]
+                ("nucleus_volume_factor", C.c_double), ("threads", C.c_int), ("average", C.c_int),
+                ("average_range", C.c_int), ("average_threshold", C.c_double)]
 
 
 _olib = None
@@ -84,7 +85,8 @@ def _p(a):
 class Oracle:
     """The C restatement of the reference step, loaded with a case's initial state."""
 
-    def __init__(self, case, counts, idx, val, cap=32, threads=0):
+    def __init__(self, case, counts, idx, val, cap=32, threads=0, nucleus_volume_factor=1.0, average_range=0,
+                 average_threshold=0.0):
         L = oracle_lib()
         self._keep = []
 
@@ -139,8 +141,9 @@ class Oracle:
                      quat=_p(quat).value if quat is not None else None, pair_sigma=_p(ps).value if ps is not None else None, pair_mu=None,
                      dg=_p(dg).value if dg is not None else None, limiting=int(case.limiting),
                      limit_phase=_p(lim).value, regularization=case.regularization, tj_factor=case.tj_factor,
-                     consider_nucleus_volume=1, nucleus_volume_factor=1.0, threads=threads,
-                     average=int(getattr(case, "average", False)))
+                     consider_nucleus_volume=1, nucleus_volume_factor=nucleus_volume_factor, threads=threads,
+                     average=int(getattr(case, "average", False)), average_range=average_range,
+                     average_threshold=average_threshold)
         self.case = case
         self.h = L.op_create(C.byref(p), cap)
         if not self.h:

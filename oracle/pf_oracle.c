@@ -721,14 +721,18 @@ static int do_increments(const op_sim* s, const entry* L, int n, pair* P)
 /* Driving-force averaging, DrivingForce::Average with $Average Yes (src/DrivingForce.cpp:242-256):
  * SetWeights (:276-291), CollectAverage (:293-383) and DistributeAverage (:384-478) in the default
  * PHASEFIELDS weights mode (:59, :137), with Range = iWidth and Threshold = iWidth/15 below an
- * interface width of 5 cells, else 1/3 (:64-73), for the per-grain driving force raw(A,B) =
+ * interface width of 5 cells, else 1/3, unless given ($Range, $Threshold; :64-73, 132-133), for the per-grain driving force raw(A,B) =
  * dG_B - dG_A that the oracle driver adds on every pair of an interface voxel.  Only the pairs of
  * positive entries have a weight; the entries of the zero-valued candidates keep weight 0, tmp 0
  * and average 0 (raw for a Seed). */
-static int df_range(const op_sim* s) { return (int)s->p.iwidth; }   /* int Range = double iWidth */
+static int df_range(const op_sim* s)
+{
+    return s->p.average_range > 0 ? s->p.average_range : (int)s->p.iwidth;   /* int Range = double iWidth */
+}
 
 static double df_threshold(const op_sim* s)
 {
+    if (s->p.average_threshold > 0.0) return s->p.average_threshold;
     return s->p.iwidth < 5.0 ? s->p.iwidth/15.0 : 1.0/3.0;
 }
 

@@ -68,6 +68,8 @@ typedef struct op_params {
     int threads;                      /* OpenMP threads (0 = runtime default)                   */
     int average;                      /* DrivingForce $Average (reference default Yes; the
                                          benchmark set-ups use No)                               */
+    int average_range;                /* $Range (0: the default, iWidth)                        */
+    double average_threshold;         /* $Threshold (0: the default)                            */
 } op_params;
 
 typedef struct op_sim op_sim;

@@ -116,3 +116,63 @@ def test_averaging_tiled_equals_generic(precision, threshold):
         got.append(ctx.download())
     r = compare_states(*got, case.ngrains)
     assert r["same_sets"] and r["max_dphi"] == 0.0, r
+
+
+def _marks(case, state, threshold):
+    """Per voxel the pair above the threshold (VolumeRatio = 1) as a key, and whether it has several."""
+    counts, idx, val = state
+    starts = np.concatenate([[0], np.cumsum(counts)])
+    key, several = np.zeros(case.n, np.int64), np.zeros(case.n, bool)
+    bar = np.sqrt(threshold * (1.0 - threshold))
+    for u in np.nonzero(counts > 1)[0]:
+        g, x = idx[starts[u]:starts[u + 1]], val[starts[u]:starts[u + 1]]
+        a, b = np.nonzero(np.triu(np.sqrt(np.outer(x, x)) > bar, 1))
+        if a.size:
+            key[u] = 1 + min(g[a[0]], g[b[0]]) * case.ngrains + max(g[a[0]], g[b[0]])
+            several[u] = a.size > 1
+    return key, several
+
+
+# One case for each way a mask is found: (case, range, threshold, what the first state has to show).
+# A tile of 8 x 8 x 16 voxels takes 4608 marks of 256 grain pairs from its halo, no voxel with several
+# pairs above the threshold, and a radius of 16; whatever is beyond that is searched voxel by voxel.
+_BOX = dict(dt=0.08, sigma=1.2, dg_scale=0.1, average=True)
+ROUTES = {
+    "range_17": (Case(20, 18, 22, 6, seed=23, iwidth=5.0, name="range_17", **_BOX), 17, 0.0, None),
+    "range_12": (Case(24, 22, 26, 8, seed=29, iwidth=5.0, name="range_12", **_BOX), 12, 0.0, None),
+    "many_marks": (Case(24, 24, 24, 30, seed=7, iwidth=6.0, name="many_marks", **_BOX), 8, 0.0,
+                   lambda m, k, s: m > 4608 and k <= 256 and not s),
+    "many_pairs": (Case(32, 32, 32, 150, seed=7, iwidth=4.0, name="many_pairs", **_BOX), 7, 0.45,
+                   lambda m, k, s: m <= 4608 and k > 256 and not s),
+    "several": (Case(24, 20, 22, 9, seed=17, iwidth=5.0, name="several", **_BOX), 0, 0.02, lambda m, k, s: s),
+}
+
+
+@pytest.mark.parametrize("name", list(ROUTES))
+def test_averaging_every_route_matches_oracle(name):
+    """Ranges, thresholds and grain sizes that send the search through each of its routes, with a nucleus
+    volume so small that every VolumeRatio is 1: the volumes' summation order plays no part."""
+    case, reach, threshold, expected = ROUTES[name]
+    state = case.initial_state()
+    factor = 0.01
+    ora = Oracle(case, *state, nucleus_volume_factor=factor, average_range=reach, average_threshold=threshold)
+    assert (ora.grains()["volume_ratio"] == 1.0).all()
+    if expected:
+        r = reach or int(case.iwidth)
+        shape = (case.nx, case.ny, case.nz)
+        key, several = _marks(case, ora.state(positive_only=True), threshold or 1.0 / 3.0)
+        at = np.ix_(*(np.arange(-r, t + r) % n for t, n in zip((8, 8, 16), shape)))
+        halo = key.reshape(shape)[at]
+        assert expected((halo > 0).sum(), np.unique(halo[halo > 0]).size, several.reshape(shape)[at].any())
+    ctx = Context(case.nx, case.ny, case.nz, iwidth=case.iwidth, stencil=case.stencil, precision="fp64", k_slots=16)
+    ctx.set_model(case.sigma_phase(), case.mu_phase(), limit=case.limit_phase(), nucleus_volume_factor=factor)
+    ctx.set_grains(case.ngrains)
+    ctx.set_driving_force(case.driving_force())
+    ctx.set_averaging(True, reach, threshold)
+    ctx.upload(*state)
+    ctx.finalize_initialization()
+    for _ in range(3):
+        assert ctx.step(case.dt, 1) & 0b11 == 0
+        ora.step(1)
+        r = compare_states(ctx.download(), ora.state(positive_only=True), case.ngrains)
+        assert r["non_borderline_mismatch_voxels"] == 0 and r["max_dphi"] <= TOL, r
