@@ -58,6 +58,55 @@ def test_tangent_state_equals_forward_and_dot_product():
     assert abs(lhs - rhs) <= 1e-10 * abs(lhs), (lhs, rhs)
 
 
+# The kinetics of grains below the reference volume (VolumeRatio < 1: scaled pairs and junction terms), of
+# triple junctions with a factor of their own, and of both; 7-point and 27-point lists (of at most 16
+# fields over the steps taken: the differentiated kernels hold no more and would report OVERFLOW_LIST)
+GENERAL = {
+    "small_grains": Case(28, 24, 26, 24, seed=7, iwidth=6.0, dt=0.08, sigma=1.2, sigma_pairs=(0.8, 0.4), dg_scale=0.05,
+                         name="small_grains"),
+    "small_grains_simple": Case(22, 26, 18, 25, seed=9, iwidth=5.0, stencil="SIMPLE", dt=0.08, sigma=1.2,
+                                sigma_pairs=(0.8, 0.4), dg_scale=0.05, tj_factor=0.2, name="small_grains_simple"),
+    "junctions": CASE.with_(tj_factor=0.3, name="junctions"),
+}
+
+
+@pytest.mark.parametrize("name", list(GENERAL))
+def test_general_kinetics_tangent_and_adjoint(name):
+    """The forward state of the tangent model is the step's (VolumeRatio = 1: bit for bit; below it the
+    volumes' summation order enters the values), the dot product agrees, and the reverse sweep of either
+    precision reproduces the stored lists.  The identity holds to the rounding of its sums (some 1e-13);
+    the volumes' summation order moves VolumeRatio by 1e-16 between the sweeps, well within the bar."""
+    case, nsteps = GENERAL[name], 8
+    G = case.ngrains
+    ctx, R, state, sig, mu, dg = _setup(case=case, nsteps=nsteps)
+    ratio = ctx.grains()["volume_ratio"]
+    assert case.tj_factor > 0 or (ratio < 1.0).sum() > G // 2
+    rng = np.random.default_rng(10)
+    w = rng.standard_normal(G)
+    ds = rng.standard_normal((G, G)); ds = (ds + ds.T) / 2; np.fill_diagonal(ds, 0)
+    dm = rng.standard_normal((G, G)); dm = (dm + dm.T) / 2; np.fill_diagonal(dm, 0)
+    dd = rng.standard_normal(G)
+    dV = R.tangent(ds, dm, dd)   # before any other step of this context
+    tangent_state = ctx.download()
+    assert ctx.stats()["status"] & 0b11 == 0
+    ref = Context.from_case(case, precision="fp64", k_slots=16, state=state)
+    ref.set_pair_table(sig, mu)
+    ref.step(case.dt, nsteps)
+    r = compare_states(tangent_state, ref.download(), G)
+    assert r["same_sets"] and r["max_dphi"] <= (0.0 if (ratio == 1.0).all() else 1e-12), r
+    R.forward()
+    gs, gm, gd = R.backward(w)
+    assert R.adjoint_status == 0
+    iu = np.triu_indices(G, 1)
+    lhs = float(w @ dV)
+    rhs = float((gs[iu] * ds[iu]).sum() + (gm[iu] * dm[iu]).sum() + gd @ dd)
+    assert abs(lhs - rhs) <= 1e-10 * abs(lhs), (lhs, rhs)
+    ctx, R, *_ = _setup(precision="fp32", case=case, nsteps=nsteps)
+    R.forward()
+    R.backward(w)
+    assert R.adjoint_status == 0
+
+
 def _fd_check(h_rel, seed, case=CASE, nsteps=T, interval=None, precision="fp64"):
     """Central differences on 32 random parameters (12 sigma pairs, 12 mu pairs, 8 driving forces)
     of L = sum_g w_g V_g(T); L is summed on the host in a fixed order (deterministic)."""
