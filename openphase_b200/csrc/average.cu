@@ -20,13 +20,16 @@
 // unless the threshold is low: then "several", resolved from the lists).  df_reach_kernel owns a
 // tile of voxels: it collects the marks of the tile and its halo once, sorted by key, so that a
 // pair of a voxel is tested against the marked voxels of its own key only (some tens) instead of
-// against the whole sphere (925 offsets at radius 6).  Blocks whose halo holds a "several" or more
-// marks or keys than their tables take, and radii above kReachRange, search the sphere directly,
-// nearest offsets first (search_sphere).
+// against the whole sphere (925 offsets at radius 6).  A tile whose halo holds a "several" or more marks
+// or keys than the tables take is left at once and listed; df_tiles_kernel searches the sphere directly
+// for the voxels of the listed tiles, nearest offsets first (search_sphere), spread over the whole
+// device.  Radii above kReachRange go to the direct search at once.
 //
 // Measured (B200, 96^3, 105 grains, radius 6, FP64, per step): the two passes over the sphere
 // 4232 + 40214 us; the direct search of every voxel about 2900 us; sorted marks 474 us, df_mark 30 us,
-// and the step itself runs on the tiled kernels (45.6 -> 0.90 ms in all).
+// and the step itself runs on the tiled kernels (45.6 -> 0.90 ms in all).  Where tables overflow (steps in
+// ms, searched by the tile's own block -> by df_tiles_kernel): radius 16 with 105 grains 84.7 -> 38.5, with
+// 30 grains 52.7 -> 21.1; 400 grains (VolumeRatio < 1: "several" in every halo), radius 6, 17.6 -> 10.4.
 #include <cfloat>
 #include <cstdint>
 
@@ -65,10 +68,12 @@ __device__ bool above(const uint8_t* __restrict__ cnt, const int16_t* __restrict
 template <class R>
 __global__ void __launch_bounds__(256) df_mark_kernel(long long N, double threshold, const uint8_t* __restrict__ cnt,
                                                        const int16_t* __restrict__ idx, const R* __restrict__ val,
-                                                       const double* __restrict__ vr, unsigned* __restrict__ strong)
+                                                       const double* __restrict__ vr, unsigned* __restrict__ strong,
+                                                       unsigned* __restrict__ tiles)
 {
     const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= N) return;
+    if (v < 2) tiles[v] = 0u;   // no tile listed, none searched
     const int c = cnt[v];
     unsigned key = 0;
     for (int b = 1; b < c; b++)
@@ -201,7 +206,11 @@ __global__ void __launch_bounds__(128) df_sphere_kernel(const __grid_constant__ 
 
 // Tile of df_reach_kernel (x, y, z) and its tables.  Halo positions are packed 10 bits an axis.
 constexpr int kReachX = 8, kReachY = 8, kReachZ = 16;
-constexpr int kReachRange = 16;     // larger radii: halos of more than 50 voxels per tile voxel
+// Largest radius the tiles are tried for.  Whether the tables hold a halo depends on how many marks it has:
+// while they do a step takes a third to a tenth of the direct search's time (96^3, radius 12: 0.9 ms against
+// 5.8 with 8 grains, 0.8 against 8.2 with 30), and where they do not it takes 0.8 to 1.13 times that time
+// (radius 13 to 16, 8 to 400 grains).  Above 16 no measured halo fits.
+constexpr int kReachRange = 16;
 constexpr int kReachMarks = 4608;   // at radius 6 a halo has 11200 voxels, some 20 % of them marked
 constexpr int kReachKeys = 256;
 
@@ -232,7 +241,7 @@ __global__ void __launch_bounds__(256) df_reach_kernel(const __grid_constant__ S
     for (int i = t; i < kReachKeys; i += NT) { key_of[i] = 0u; first[i] = 0; filled[i] = 0; }
     if (t == 0) { entries = 0; failed = 0; }
     __syncthreads();
-    for (int i = t; i < hx * hy * hz; i += NT)
+    for (int i = t; i < hx * hy * hz && !*(volatile int*)&failed; i += NT)
     {
         const int iz = i % hz, iy = (i / hz) % hy, ix = i / (hz * hy);
         const long long u = (long long)wrap_axis(x0 - r + ix, p.nx) * plane + wrap_axis(y0 - r + iy, p.ny) * p.nz
@@ -255,14 +264,9 @@ __global__ void __launch_bounds__(256) df_reach_kernel(const __grid_constant__ S
         slot_of[e] = (uint8_t)h;
     }
     __syncthreads();
-    const int x = x0, y = y0;
     if (failed)
     {
-        for (int i = t; i < kReachX * kReachY * kReachZ; i += NT)
-        {
-            const int vz = z0 + i % kReachZ, vy = y + (i / kReachZ) % kReachY, vx = x + i / (kReachZ * kReachY);
-            if (vx < p.nx && vy < p.ny && vz < p.nz) search_sphere<R>(p, aa, cnt, idx, val, vr, vx, vy, vz);
-        }
+        if (t == 0) aa.tiles[2u + atomicAdd(&aa.tiles[0], 1u)] = (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
         return;
     }
     if (t < 32)
@@ -294,7 +298,7 @@ __global__ void __launch_bounds__(256) df_reach_kernel(const __grid_constant__ S
     for (int i = t; i < kReachX * kReachY * kReachZ; i += NT)
     {
         const int iz = i % kReachZ, iy = (i / kReachZ) % kReachY, ix = i / (kReachZ * kReachY);
-        const int vx = x + ix, vy = y + iy, vz = z0 + iz;
+        const int vx = x0 + ix, vy = y0 + iy, vz = z0 + iz;
         if (vx >= p.nx || vy >= p.ny || vz >= p.nz) continue;
         const long long v = (long long)vx * plane + vy * p.nz + vz;
         const int c = cnt[v];
@@ -331,27 +335,64 @@ __global__ void __launch_bounds__(256) df_reach_kernel(const __grid_constant__ S
     }
 }
 
+// The direct search for the tiles that df_reach_kernel listed (gy, gx: tiles along y and z).  How long a
+// voxel searches depends on where it lies, so that the warps fetch 32 voxels at a time.
+template <class R>
+__global__ void __launch_bounds__(128) df_tiles_kernel(const __grid_constant__ StepParams p, AvgArrays aa, unsigned gy,
+                                                        unsigned gx, const uint8_t* __restrict__ cnt,
+                                                        const int16_t* __restrict__ idx, const R* __restrict__ val,
+                                                        const double* __restrict__ vr)
+{
+    constexpr unsigned kParts = kReachX * kReachY * kReachZ / 32;
+    const unsigned items = aa.tiles[0] * kParts, lane = threadIdx.x & 31u;
+    while (true)
+    {
+        unsigned item = lane == 0 ? atomicAdd(&aa.tiles[1], 1u) : 0u;
+        item = __shfl_sync(0xffffffffu, item, 0);
+        if (item >= items) return;
+        const unsigned tile = aa.tiles[2u + item / kParts], i = (item % kParts) * 32u + lane;
+        const int x = (int)(tile / (gx * gy) * kReachX + i / (kReachZ * kReachY));
+        const int y = (int)(tile / gx % gy * kReachY + i / kReachZ % kReachY);
+        const int z = (int)(tile % gx * kReachZ + i % kReachZ);
+        if (x < p.nx && y < p.ny && z < p.nz) search_sphere<R>(p, aa, cnt, idx, val, vr, x, y, z);
+        __syncwarp();
+    }
+}
+
 template <class R>
 int launch_average_of(const StepParams& p, const AvgArrays& aa, const uint8_t* cnt, const int16_t* idx, const R* val,
-                      const double* vr, cudaStream_t s)
+                      const double* vr, cudaStream_t s, int* kernels)
 {
-    df_mark_kernel<R><<<(unsigned)((p.n + 255) / 256), 256, 0, s>>>(p.n, aa.weight_threshold, cnt, idx, val, vr, aa.strong);
+    df_mark_kernel<R><<<(unsigned)((p.n + 255) / 256), 256, 0, s>>>(p.n, aa.weight_threshold, cnt, idx, val, vr, aa.strong,
+                                                                  aa.tiles);
     const dim3 tiles((p.nz + kReachZ - 1) / kReachZ, (p.ny + kReachY - 1) / kReachY, (p.nx + kReachX - 1) / kReachX);
     if (aa.range <= kReachRange && tiles.y <= 65535u && tiles.z <= 65535u)
+    {
         df_reach_kernel<R><<<tiles, 256, 0, s>>>(p, aa, cnt, idx, val, vr);
+        df_tiles_kernel<R><<<148 * 16, 128, 0, s>>>(p, aa, tiles.y, tiles.x, cnt, idx, val, vr);
+        *kernels += 3;
+    }
     else
+    {
         df_sphere_kernel<R><<<(unsigned)((p.n + 127) / 128), 128, 0, s>>>(p, aa, cnt, idx, val, vr);
+        *kernels += 2;
+    }
     return (int)cudaGetLastError();
 }
 
 }  // namespace
 
+size_t average_tiles(int nx, int ny, int nz)
+{
+    return (size_t)((nx + kReachX - 1) / kReachX) * ((ny + kReachY - 1) / kReachY) * ((nz + kReachZ - 1) / kReachZ);
+}
+
 int launch_average(const StepParams& p, const AvgArrays& aa, const uint8_t* cnt, const int16_t* idx,
-                   const void* val, bool fp32, const double* vr, void* stream)
+                   const void* val, bool fp32, const double* vr, void* stream, int* kernels)
 {
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    return fp32 ? launch_average_of<float>(p, aa, cnt, idx, static_cast<const float*>(val), vr, s)
-                : launch_average_of<double>(p, aa, cnt, idx, static_cast<const double*>(val), vr, s);
+    return fp32 ? launch_average_of<float>(p, aa, cnt, idx, static_cast<const float*>(val), vr, s, kernels)
+                : launch_average_of<double>(p, aa, cnt, idx, static_cast<const double*>(val), vr, s, kernels);
 }
 
 }  // namespace opgpu

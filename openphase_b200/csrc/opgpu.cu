@@ -107,7 +107,7 @@ struct opgpu_ctx {
     bool averaging = false;
     int avg_range = 0;
     double avg_threshold = 0.0;
-    unsigned *d_avg_strong = nullptr, *d_avg_mask = nullptr;
+    unsigned *d_avg_strong = nullptr, *d_avg_mask = nullptr, *d_avg_tiles = nullptr;
     char4* d_avg_off = nullptr;      // sphere offsets, nearest first
     int avg_noff = 0;
 };
@@ -692,7 +692,7 @@ extern "C" uint32_t opgpu_destroy(opgpu_ctx* ctx)
     dfree(ctx->d_wl);
     dfree(ctx->d_bucket); dfree(ctx->d_bucket_count); dfree(ctx->d_bucket_off);
     dfree(ctx->d_facets);
-    dfree(ctx->d_avg_strong); dfree(ctx->d_avg_mask); dfree(ctx->d_avg_off);
+    dfree(ctx->d_avg_strong); dfree(ctx->d_avg_mask); dfree(ctx->d_avg_tiles); dfree(ctx->d_avg_off);
     dfree(ctx->d_status);
     pinned_free(ctx->h_stage, ctx->h_stage_bytes);
     dfree(ctx->d_counters);
@@ -995,6 +995,8 @@ extern "C" uint32_t opgpu_set_averaging(opgpu_ctx* ctx, int32_t enable, int32_t 
     CK(cudaMemcpy(ctx->d_avg_off, off.data(), off.size() * sizeof(char4), cudaMemcpyHostToDevice));
     if (!ctx->d_avg_strong) CK(dalloc(&ctx->d_avg_strong, (size_t)ctx->n));
     if (!ctx->d_avg_mask) CK(dalloc(&ctx->d_avg_mask, (size_t)ctx->n * kAvgWords));
+    if (!ctx->d_avg_tiles)
+        CK(dalloc(&ctx->d_avg_tiles, 2 + average_tiles(ctx->grid.nx, ctx->grid.ny, ctx->grid.nz)));
     ctx->avg_noff = (int)off.size();
     ctx->avg_range = R;
     ctx->avg_threshold = t;
@@ -1280,12 +1282,13 @@ static uint32_t enqueue_steps(opgpu_ctx* ctx, double dt, int nsteps, bool partia
         if (ctx->averaging && sp.use_dg)
         {
             // DrivingForce::Average on the state the step starts from
-            const AvgArrays aa{ctx->d_avg_strong, ctx->d_avg_mask, ctx->d_avg_off, ctx->avg_noff, ctx->avg_range,
-                               std::sqrt(ctx->avg_threshold * (1.0 - ctx->avg_threshold))};
+            const AvgArrays aa{ctx->d_avg_strong, ctx->d_avg_mask, ctx->d_avg_tiles, ctx->d_avg_off, ctx->avg_noff,
+                               ctx->avg_range, std::sqrt(ctx->avg_threshold * (1.0 - ctx->avg_threshold))};
+            int kernels = 0;
             const int rc = launch_average(sp, aa, ctx->cnt[in], ctx->idx[in], ctx->val[in], ctx->fp32 != 0, ctx->d_vr,
-                                          ctx->stream);
+                                          ctx->stream, &kernels);
             if (rc != 0) return fail(ctx, OPGPU_E_CUDA, std::string("averaging: ") + cudaGetErrorString((cudaError_t)rc));
-            ctx->kernel_launches += 2;   // mark, reach
+            ctx->kernel_launches += kernels;
             a.avg_mask = ctx->d_avg_mask;
         }
         set_worklists(ctx, a);

@@ -10,6 +10,7 @@
 // A voxel's interface flag is never stored: flag = 2 if cnt > 1, else 1 if any of its 26 periodic
 // neighbours has cnt > 1, else 0 (identical to NodePF::finalize + PhaseField::SetFlagsSR).
 #pragma once
+#include <stddef.h>
 #include <stdint.h>
 
 #include <vector_types.h>
@@ -37,6 +38,8 @@ constexpr int kAvgWords = 4;     // 120 pairs of 16 stored fields
 struct AvgArrays {
     unsigned* strong;            // [N] key of the voxel's pair above the threshold
     unsigned* mask;              // [kAvgWords][N]
+    unsigned* tiles;             // [2 + average_tiles] the tiles searched directly: their number, the next item
+                                 // of work, the tiles
     const char4* offsets;        // [noff] sphere offsets with Range - |d| > 0, nearest first
     int noff;
     int range;
@@ -210,9 +213,11 @@ int launch_step_f32(const StepParams& p, const StepArrays& a, int k_slots, int v
 // The classify kernel of the tiled step alone; returns the number of classify blocks or < 0.
 int launch_classify_f64(const StepParams& p, const StepArrays& a, void* stream);
 int launch_classify_f32(const StepParams& p, const StepArrays& a, void* stream);
-// Driving-force averaging of a state (average.cu): writes aa.strong and aa.mask.
+// Driving-force averaging of a state (average.cu): writes aa.strong, aa.mask and aa.tiles; adds its launches
+// to *kernels.
+size_t average_tiles(int nx, int ny, int nz);
 int launch_average(const StepParams& p, const AvgArrays& aa, const uint8_t* cnt, const int16_t* idx,
-                   const void* val, bool fp32, const double* vr, void* stream);
+                   const void* val, bool fp32, const double* vr, void* stream, int* kernels);
 // Add the volumes of the window planes of a state to vol_acc (defined in step_f64.cu).
 int launch_volume_recount(const StepParams& p, const uint8_t* cnt, const int16_t* idx, const void* val, int fp32,
                           double* vol_acc, void* stream);
