@@ -1308,39 +1308,41 @@ int launch_tlm_step(const StepParams& p, const StepArrays& a, const AdjArrays& a
 constexpr int kAdjListBlocks = 148 * 32;   // blocks of each per-length adjoint kernel
 
 // The per-length kernels, the worklist kernel (few voxels, each a long serial chain: its own stream)
-// and the bulk kernel write disjoint voxels and run beside each other; each is a latency chain on
-// small grids (56 x 60 x 50, FP64: 51, 109, 136, 115, 130, 172, 228 us for N = 2..8, worklist
-// 533 us).
+// and the bulk kernel write disjoint voxels.  Each per-length kernel is a latency chain on small grids
+// (56 x 60 x 50, FP64: 51, 109, 136, 115, 130, 172, 228 us for N = 2..8, worklist 533 us) and they run
+// beside each other there; with `lists_beside` false only the worklist kernel has another stream.
 template <class R, int KS>
 static void adjoint_kernels(const StepParams& p, const StepArrays& a, const AdjArrays& aa, int nblocks,
-                            const SideFork& fork)
+                            const SideFork& fork, bool lists_beside)
 {
     const cudaStream_t s = fork.main;
+    auto on = [&](int k) { return lists_beside ? fork.on(k) : s; };
     adjoint_worklist_kernel<R, KS><<<148 * 8, 64, 0, fork.on(2)>>>(p, a, aa);
-    adjoint_list_kernel<R, 8><<<kAdjListBlocks, 128, 0, fork.on(0)>>>(p, a, aa, nblocks);
-    adjoint_list_kernel<R, 7><<<kAdjListBlocks, 128, 0, fork.on(1)>>>(p, a, aa, nblocks);
+    adjoint_list_kernel<R, 8><<<kAdjListBlocks, 128, 0, on(0)>>>(p, a, aa, nblocks);
+    adjoint_list_kernel<R, 7><<<kAdjListBlocks, 128, 0, on(1)>>>(p, a, aa, nblocks);
     adjoint_list_kernel<R, 6><<<kAdjListBlocks, 128, 0, s>>>(p, a, aa, nblocks);
-    adjoint_list_kernel<R, 5><<<kAdjListBlocks, 128, 0, fork.on(3)>>>(p, a, aa, nblocks);
+    adjoint_list_kernel<R, 5><<<kAdjListBlocks, 128, 0, on(3)>>>(p, a, aa, nblocks);
     adjoint_list_kernel<R, 4><<<kAdjListBlocks, 128, 0, s>>>(p, a, aa, nblocks);
-    adjoint_list_kernel<R, 3><<<kAdjListBlocks, 128, 0, fork.on(3)>>>(p, a, aa, nblocks);
-    adjoint_list_kernel<R, 2><<<kAdjListBlocks, 128, 0, fork.on(1)>>>(p, a, aa, nblocks);
+    adjoint_list_kernel<R, 3><<<kAdjListBlocks, 128, 0, on(3)>>>(p, a, aa, nblocks);
+    adjoint_list_kernel<R, 2><<<kAdjListBlocks, 128, 0, on(1)>>>(p, a, aa, nblocks);
     adjoint_bulk_kernel<<<grid_of(p.n, 256), 256, 0, s>>>(p, a.cnt_in, aa);
 }
 
 int launch_adjoint_step(const StepParams& p, const StepArrays& a, const AdjArrays& aa, int k_slots, bool fp32,
-                        int nblocks, double* lam0, void* stream, const SideStreams& side)
+                        int nblocks, double* lam0, void* stream, const SideStreams& side, unsigned worklist)
 {
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const SideFork fork(&side, s);
+    const SideFork fork(worklist < kListsBeside ? &side : nullptr, s);
+    const bool beside = worklist < kAdjointListsBeside;
     bool known = true;
     switch (k_slots * 2 + (fp32 ? 1 : 0))
     {
-        case 16: adjoint_kernels<double, 8>(p, a, aa, nblocks, fork); break;
-        case 17: adjoint_kernels<float, 8>(p, a, aa, nblocks, fork); break;
-        case 24: adjoint_kernels<double, 12>(p, a, aa, nblocks, fork); break;
-        case 25: adjoint_kernels<float, 12>(p, a, aa, nblocks, fork); break;
-        case 32: adjoint_kernels<double, 16>(p, a, aa, nblocks, fork); break;
-        case 33: adjoint_kernels<float, 16>(p, a, aa, nblocks, fork); break;
+        case 16: adjoint_kernels<double, 8>(p, a, aa, nblocks, fork, beside); break;
+        case 17: adjoint_kernels<float, 8>(p, a, aa, nblocks, fork, beside); break;
+        case 24: adjoint_kernels<double, 12>(p, a, aa, nblocks, fork, beside); break;
+        case 25: adjoint_kernels<float, 12>(p, a, aa, nblocks, fork, beside); break;
+        case 32: adjoint_kernels<double, 16>(p, a, aa, nblocks, fork, beside); break;
+        case 33: adjoint_kernels<float, 16>(p, a, aa, nblocks, fork, beside); break;
         default: known = false; break;
     }
     const cudaError_t e = fork.join();

@@ -39,9 +39,10 @@ int launch_tlm_step(const StepParams& p, const StepArrays& a, const AdjArrays& a
 // and its adjoint; the classify kernel has just run on the state before the step (its work
 // records, buckets and worklist in a; nblocks its block count).  Writes the adjoint of the state
 // before the step to lam0 and accumulates the parameter gradients.
-// The list-length kernels and the worklist kernel run beside each other on `side`.
+// `worklist`, the length of the general-path worklist as last known, decides which of the kernels run
+// beside each other on `side`.
 int launch_adjoint_step(const StepParams& p, const StepArrays& a, const AdjArrays& aa, int k_slots, bool fp32,
-                        int nblocks, double* lam0, void* stream, const SideStreams& side);
+                        int nblocks, double* lam0, void* stream, const SideStreams& side, unsigned worklist);
 // lam[s][v] = dLdV[idx[s][v]] on the stored entries (adjoint of a loss on the grain volumes).
 int launch_lambda_init(long long n, const uint8_t* cnt, const int16_t* idx, const double* dLdV, double* lam,
                        void* stream);

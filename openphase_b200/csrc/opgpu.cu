@@ -74,12 +74,12 @@ struct opgpu_ctx {
     std::vector<double> h_dg;           // [G] driving forces given to opgpu_set_driving_force
     std::vector<double> h_dg_pair;      // [G*G] host side of the limited driving-force table
     bool pair_energy_dirty = true;
-    uint32_t* d_status = nullptr;
-    unsigned char* h_stage = nullptr;   // pinned: the status word, then the grain records on their way out
+    uint32_t* d_status = nullptr;       // status word, length of the general-path worklist
+    unsigned worklist = 0;              // that length as the host last read it
+    unsigned char* h_stage = nullptr;   // pinned: the two words, then the grain records on their way out
     size_t h_stage_bytes = 0;
     unsigned long long* d_counters = nullptr;
     int* d_slow_list = nullptr;      // overflow worklist of the tiled kernel (capacity N)
-    unsigned* d_slow_count = nullptr;
     // work buffer of the classify / compute split (see tile_kernel.cuh)
     unsigned char* d_wl = nullptr;
     long long wl_slice = 0;
@@ -559,10 +559,11 @@ uint32_t read_status(opgpu_ctx* ctx)
 {
     if (!reserve_stage(ctx, 0)) return fail(ctx, OPGPU_E_CUDA, "no pinned memory for the status word");
     uint32_t* word = reinterpret_cast<uint32_t*>(ctx->h_stage);
-    CK(cudaMemcpyAsync(word, ctx->d_status, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaMemcpyAsync(word, ctx->d_status, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaMemsetAsync(ctx->d_status, 0, sizeof(uint32_t), ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
-    const uint32_t st = *word;
+    const uint32_t st = word[0];
+    ctx->worklist = word[1];
     for (size_t i = 0; i < ctx->ev_used; i++)
     {
         float ms = 0.f, ms_c = 0.f;
@@ -641,7 +642,6 @@ extern "C" uint32_t opgpu_create(const opgpu_grid* grid, opgpu_ctx** out)
         if (cudaMemset(ctx->cnt[b], 0, (size_t)ctx->n) != cudaSuccess) return bail(OPGPU_E_CUDA);
     }
     if (dalloc(&ctx->d_slow_list, (size_t)ctx->n) != cudaSuccess) return bail(OPGPU_E_CUDA);
-    if (dalloc(&ctx->d_slow_count, 1) != cudaSuccess) return bail(OPGPU_E_CUDA);
     {
         int xchunk = 0, gz = 0, gy = 0, gx = 0;
         tiled_geometry(g.nx, g.ny, g.nz, (int)ctx->rsz, &xchunk, &gz, &gy, &gx);
@@ -658,9 +658,11 @@ extern "C" uint32_t opgpu_create(const opgpu_grid* grid, opgpu_ctx** out)
         if (cudaMemset(ctx->d_bucket_off, 0, (kListCap + 1) * (nblocks + 1) * sizeof(unsigned)) != cudaSuccess)
             return bail(OPGPU_E_CUDA);
     }
-    if (dalloc(&ctx->d_status, 1) != cudaSuccess) return bail(OPGPU_E_CUDA);
+    if (dalloc(&ctx->d_status, 2) != cudaSuccess) return bail(OPGPU_E_CUDA);
     if (dalloc(&ctx->d_counters, kNumCounters) != cudaSuccess) return bail(OPGPU_E_CUDA);
-    cudaMemset(ctx->d_status, 0, sizeof(uint32_t));
+    ctx->worklist = worklist_guess(ctx->n);
+    const uint32_t words[2] = {0u, ctx->worklist};
+    if (cudaMemcpy(ctx->d_status, words, sizeof(words), cudaMemcpyHostToDevice) != cudaSuccess) return bail(OPGPU_E_CUDA);
     cudaMemset(ctx->d_counters, 0, kNumCounters * sizeof(unsigned long long));
     StepParams& sp = ctx->sp;
     sp.nx = g.nx; sp.ny = g.ny; sp.nz = g.nz; sp.n = ctx->n;
@@ -688,7 +690,6 @@ extern "C" uint32_t opgpu_destroy(opgpu_ctx* ctx)
     free_grains(ctx);
     for (cudaEvent_t e : ctx->ev_pool) cudaEventDestroy(e);
     dfree(ctx->d_slow_list);
-    dfree(ctx->d_slow_count);
     dfree(ctx->d_wl);
     dfree(ctx->d_bucket); dfree(ctx->d_bucket_count); dfree(ctx->d_bucket_off);
     dfree(ctx->d_facets);
@@ -1252,7 +1253,7 @@ extern "C" uint32_t opgpu_finalize_initialization(opgpu_ctx* ctx)
 // The classify kernel's work records, buckets and worklist.
 static void set_worklists(const opgpu_ctx* ctx, StepArrays& a)
 {
-    a.slow_list = ctx->d_slow_list; a.slow_count = ctx->d_slow_count; a.slow_cap = (unsigned)ctx->n;
+    a.slow_list = ctx->d_slow_list; a.slow_count = ctx->d_status + 1; a.slow_cap = (unsigned)ctx->n;
     a.wl = ctx->d_wl; a.wl_slice = ctx->wl_slice;
     a.bucket = ctx->d_bucket; a.bucket_count = ctx->d_bucket_count; a.bucket_off = ctx->d_bucket_off;
     a.bucket_cap = ctx->bucket_cap; a.slice = ctx->slice;
@@ -1294,6 +1295,7 @@ static uint32_t enqueue_steps(opgpu_ctx* ctx, double dt, int nsteps, bool partia
         set_worklists(ctx, a);
         LaunchInfo info;
         info.side = &ctx->side;
+        info.worklist = ctx->worklist;
         if (ctx->timing)
         {
             if (ctx->ev_pool.size() < 3 * (ctx->ev_used + 1))
@@ -1794,7 +1796,7 @@ extern "C" uint32_t opgpu_adjoint_step(opgpu_ctx* ctx, int32_t slot, double dt)
     CK(cudaMemsetAsync(ctx->d_vol_acc, 0, (size_t)ctx->G * sizeof(double), ctx->stream));
     CK(cudaMemsetAsync(ctx->d_counters, 0, 3 * sizeof(unsigned long long), ctx->stream));   // wide, entries in/out
     CK(cudaMemsetAsync(ctx->d_counters + kCntCrowdedLast, 0, sizeof(unsigned long long), ctx->stream));
-    if (launch_adjoint_step(sp, a, aa, ctx->K, ctx->fp32 != 0, nblocks, lam0, ctx->stream, ctx->side))
+    if (launch_adjoint_step(sp, a, aa, ctx->K, ctx->fp32 != 0, nblocks, lam0, ctx->stream, ctx->side, ctx->worklist))
         return fail(ctx, OPGPU_E_CUDA, "opgpu_adjoint_step: launch");
     ctx->kernel_launches += 12;
     ctx->lam_cur = 1 - ctx->lam_cur;

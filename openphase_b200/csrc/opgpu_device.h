@@ -196,11 +196,40 @@ struct SideStreams {
     void* join[kSideStreams] = {};     // cudaEvent_t
 };
 
+// Which kernels of a step run beside each other goes by the length of the general-path worklist, as the
+// host last read it (with the status word).  All write disjoint voxels; the order changes no result.
+// Each per-length kernel is a chain of dependent arithmetic and instruction fetches whose length hardly
+// depends on its entry count on small grids (64^3, FP64: 17, 19, 26, 34, 54, 77, 115 us for N = 2..8), so
+// that they gain from each other's company until each fills the device.  The general path has the
+// opposite: it gathers from the whole neighbourhood, and once it runs long the lists beside it cost it
+// its cache.  Step in us, one after another / lists beside each other / general path beside them (mean
+// grain volume, worklist):
+//   FP64  64^3 8389       <1 k   289   183   149      FP32  64^3 8389       <1 k   290   178   143
+//         128^3 8389       4 k   842   638   621            128^3 8389       4 k   801   593   582
+//         192^3 8389      14 k  1921  1765  1832            192^3 8389      14 k  1753  1623  1632
+//         256^3 8389      29 k  4073  4028  4133            256^3 8389      29 k  3771  3708  3748
+//         128^3 3500      31 k  1485  1344  1466            128^3 3500      31 k  1371  1234  1261
+//         64^3 1728       47 k   985   931   950            160^3 3500      61 k  2227  2093  2300
+//         240^3 5000      83 k  5016  5008  5623            240^3 5000      83 k  4680  4831  4832
+//         224^3 3500     180 k  7065  7419  8199            224^3 3500     180 k  6313  6758  7310
+//         96^3 1728      170 k  2927  3008  3383            96^3 1728      100 k  2118  2255  2296
+// The adjoint's lists (one after another / worklist kernel beside them / all beside each other, us):
+//   FP64 96^3 8192 2 k 2573 2259 2167; 96^3 4000 9 k 5127 5009 5267; 128^3 8192 4 k 2969 2641 2779;
+//   192^3 8192 14 k 7365 7105 7464; 224^3 4000 120 k 20409 20588 21262; 256^3 4000 180 k 34234 36768 39128.
+// The tangent step gains with all of them beside each other at every size (96^3 1924 -> 1145, 256^3 17141 ->
+// 16183).
+constexpr unsigned kGeneralBeside = 10000;      // below: the general path beside the lists
+constexpr unsigned kListsBeside = 80000;        // below: the lists beside each other
+constexpr unsigned kAdjointListsBeside = 2500;  // below: the adjoint's lists beside each other
+// Before a first step: the worklist of grains of some 8400 voxels.
+inline unsigned worklist_guess(long long n) { return (unsigned)(n / 500); }
+
 // Filled by the launchers: kernels launched, and an event recorded after the classify kernel
 // (when `after_classify` is not null) so the caller can time it separately.
 struct LaunchInfo {
     void* after_classify = nullptr;   // cudaEvent_t
     const SideStreams* side = nullptr;   // null: every kernel on the context's stream
+    unsigned worklist = 0;            // length of the general-path worklist, as last known
     int kernels = 0;
 };
 

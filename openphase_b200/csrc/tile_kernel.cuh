@@ -1205,14 +1205,7 @@ struct SideFork {
     }
 };
 
-// The per-length kernels and the general path write disjoint voxels, so they run beside each other.
-// On small grids each is a chain of dependent arithmetic and instruction fetches whose length hardly
-// depends on the entry count (64^3, FP64: 17, 19, 26, 34, 54, 77, 115 us for N = 2..8), so the chains
-// are dealt out to streams of about equal length, the longest alone.  On large grids every kernel fills
-// the device and only the tails overlap, while the mixed resident blocks cost cache hits.  Step, one
-// stream -> side streams (FP64, us): 64^3 337 -> 192, 128^3 1024 -> 794, 192^3 2520 -> 2355, 224^3
-// 3749 -> 3690, 256^3 5465 -> 5600: the line lies between the last two.
-constexpr long long kSideVoxels = 12000000;
+// The per-length kernels, dealt out to streams of about equal length (64^3: the longest alone).
 template <class R, bool AVG>
 void launch_lists(const StepParams& p, const StepArrays& a, int cb, int nblocks, const SideFork& fork)
 {
@@ -1254,7 +1247,10 @@ int launch_tiled_ns(const StepParams& p, const StepArrays& a, void* stream, Laun
     }
     bucket_scan_kernel<<<kListCap - 1, 1024, 0, s>>>(a, nblocks);
     const int cb = compute_blocks(p.n);
-    const SideFork fork(info && p.n <= kSideVoxels ? info->side : nullptr, s);
+    const bool lists_beside = info && info->side && info->worklist < kListsBeside;
+    const bool general_beside = lists_beside && info->worklist < kGeneralBeside;
+    if (!p.aniso && !general_beside) gk<<<148 * 4, 128, wsm, s>>>(p, a);
+    const SideFork fork(lists_beside ? info->side : nullptr, s);
     if (p.aniso)
     {
         aniso_worklist_kernel<R, KS, KL><<<148 * 8, 64, 0, fork.on(0)>>>(p, a);
@@ -1262,7 +1258,7 @@ int launch_tiled_ns(const StepParams& p, const StepArrays& a, void* stream, Laun
     }
     else
     {
-        gk<<<148 * 4, 128, wsm, fork.on(2)>>>(p, a);
+        if (general_beside) gk<<<148 * 4, 128, wsm, fork.on(2)>>>(p, a);
         if (a.avg_mask) launch_lists<R, true>(p, a, cb, nblocks, fork);
         else launch_lists<R, false>(p, a, cb, nblocks, fork);
     }

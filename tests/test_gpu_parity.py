@@ -219,3 +219,31 @@ def test_single_grain_and_tiny_grids_are_stable():
         assert np.max(np.abs(va - vb)) <= 1e-12
         r = compare_states((ca, ia, va), ora.state(positive_only=True), tiny.ngrains)
         assert r["non_borderline_mismatch_voxels"] == 0 and r["max_dphi"] <= 1e-9, r
+
+
+# (grid, mean grain volume, general-path voxels a step has to take): every order of a step's kernels, which
+# goes by that number -- beside each other, the general path first, one after another
+ORDERS = {"beside": (40, 3500, (100, 10000)), "general_first": (64, 2200, (10000, 80000)), "in_turn": (96, 1728, (80000, 10 ** 9))}
+
+
+@pytest.mark.parametrize("name", list(ORDERS))
+def test_every_order_of_the_kernels_equals_generic(name):
+    side, volume, (low, high) = ORDERS[name]
+    case = Case(side, side, side, side ** 3 // volume, seed=2, iwidth=6.0, dt=0.08, sigma=1.2, sigma_pairs=(0.8, 0.4),
+                dg_scale=0.05, name=name)
+    state = case.initial_state()
+    got = []
+    for variant in ("tiled", "generic"):
+        ctx = Context.from_case(case, precision="fp64", k_slots=16, state=state)
+        ctx.set_kernel_variant(variant)
+        taken = []
+        for steps in (4, 1, 1):   # the order of a call goes by the step before it
+            before = ctx.stats()["general_path_total"]
+            assert ctx.step(case.dt, steps) & 0b11 == 0
+            taken.append((ctx.stats()["general_path_total"] - before) / steps)
+        if variant == "tiled":
+            assert all(low <= t < high for t in taken[1:]), taken
+        got.append(ctx.download())
+    r = compare_states(*got, case.ngrains)
+    # VolumeRatio < 1 in places: the volumes' summation order
+    assert r["same_sets"] and r["max_dphi"] <= 1e-12, r
