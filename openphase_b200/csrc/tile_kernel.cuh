@@ -670,6 +670,7 @@ static __global__ void __launch_bounds__(1024) bucket_scan_kernel(const StepArra
     if (t == 0) off[nslices] = s_warp[31];
 }
 
+constexpr int kTogetherShare = 48;   // (see list_compute_kernel)
 constexpr int kChunkTable = 128;   // 32-entry chunks of a compute block whose slices are tabulated
 constexpr int kVolCache = 2;       // per-thread grain-volume cache of the compute kernels (four entries, of
                                    // which a thread's few voxels fill most once: FP32 step 4072 -> 4002 us)
@@ -686,13 +687,23 @@ constexpr int kVolCache = 2;       // per-thread grain-volume cache of the compu
 // 396 283 185 147 us to 235 391 452 305 219 131 129 (233 389 412 281 206 126 117 with the block bounds and the
 // smaller volume cache below).
 //
+// The kinetics have two branches, for lists whose grains all have their reference volume and for the
+// others.  Each is a long straight line, fetched once by the warps that run it at about the same time;
+// where small grains mix the two, warps in different branches fetch for themselves (128^3, mean grain
+// 1728 voxels, FP32, N = 6: 13.5 of 22 cycles an instruction wait for it).  With `together` a block's
+// warps take one branch in step: the general one if any list needs it, which gives a full list the same
+// values.  N = 5, 6, 7, FP32: 227 400 338 -> 184 296 251 us, FP64: 228 364 208 -> 191 268 208; the step
+// at 160^3 5.76 -> 4.89 and 7.98 -> 7.31 ms.  With grains of 8400 voxels the barrier costs a 256^3 step
+// about 1 %, so that it goes by the share of the voxels on the general path (kTogetherShare: more than
+// 3 % with grains of 1728 voxels, 0.2 % to 1.7 % with 3500, 0.2 % with 8400).
+//
 // N <= kListCap <= the stored fields per voxel, so a new record always fits.  AVG: averaged driving
 // forces (a template parameter: the mask costs the plain step registers).
 // Resident blocks: six for N <= 3, five for 4 and 5, three beyond (the registers each takes unbounded
 // allow five, four and two to three): FP64 step at 256^3 4365 -> 4298 us.
 template <class R, int N, bool AVG>
 __global__ void __launch_bounds__(128, N <= 3 ? 6 : (N <= 5 ? 5 : 3)) list_compute_kernel(const __grid_constant__ StepParams p, const StepArrays a,
-                                                           int nslices)
+                                                           int nslices, bool together)
 {
     constexpr int NP = N * (N - 1) / 2;
     __shared__ int s_key[kTileVolSlots];
@@ -729,14 +740,13 @@ __global__ void __launch_bounds__(128, N <= 3 ? 6 : (N <= 5 ? 5 : 3)) list_compu
     R* __restrict__ vout = static_cast<R*>(a.val_out);
     uint32_t st = 0;
     unsigned eout = 0;
-    const unsigned lane = t & 31u;
-    for (unsigned base = r0 + (t - lane); base < r1; base += blockDim.x)   // the same trip count per warp
+    for (unsigned first = r0; first < r1; first += blockDim.x)   // the same trip count for the block's warps
     {
-        const unsigned e = base + lane;
-        // slice of the warp's first entry, then of each lane's entry
-        int lo = tabulated ? s_chunk[(base - r0) >> 5] : slice_of(off, nslices, base);
-        if (e < r1)
-        {
+        // (the lanes beyond the last entry repeat it and store nothing)
+        const bool mine = first + t < r1;
+        const unsigned e = mine ? first + t : r1 - 1u;
+        // slice of the first entry of this one's chunk of 32, then its own
+        int lo = tabulated ? s_chunk[(e - r0) >> 5] : slice_of(off, nslices, r0 + ((e - r0) & ~31u));
         while (off[lo + 1] <= e) lo++;   // off[nslices] = total > e
         const int2 ent = buck[(long long)lo * a.slice + (e - off[lo])];
         const unsigned char* __restrict__ wbase = a.wl + (long long)lo * a.wl_slice;
@@ -762,6 +772,7 @@ __global__ void __launch_bounds__(128, N <= 3 ? 6 : (N <= 5 ? 5 : 3)) list_compu
             vr[k] = a.vr[g[k]];
             full = full && vr[k] == 1.0;
         }
+        if (together) full = __syncthreads_and(full);
         R sg[NP];
 #pragma unroll
         for (int i = 0; i < N; i++)
@@ -1011,6 +1022,7 @@ __global__ void __launch_bounds__(128, N <= 3 ? 6 : (N <= 5 ? 5 : 3)) list_compu
         }
         const double norm = 1.0 / total;
         int pos = 0;
+        if (!mine) continue;
 #pragma unroll
         for (int i = 0; i < N; i++)
         {
@@ -1044,7 +1056,6 @@ __global__ void __launch_bounds__(128, N <= 3 ? 6 : (N <= 5 ? 5 : 3)) list_compu
         if (m == 0) st |= kStEmptyVoxel;
         a.cnt_out[v] = (uint8_t)pos;
         eout += pos;
-        }
     }
 #pragma unroll
     for (int c = 0; c < kVolCache; c++)
@@ -1207,16 +1218,16 @@ struct SideFork {
 
 // The per-length kernels, dealt out to streams of about equal length (64^3: the longest alone).
 template <class R, bool AVG>
-void launch_lists(const StepParams& p, const StepArrays& a, int cb, int nblocks, const SideFork& fork)
+void launch_lists(const StepParams& p, const StepArrays& a, int cb, int nblocks, const SideFork& fork, bool together)
 {
     const cudaStream_t s = fork.main;
-    list_compute_kernel<R, 8, AVG><<<cb, 128, 0, fork.on(0)>>>(p, a, nblocks);
-    list_compute_kernel<R, 7, AVG><<<cb, 128, 0, fork.on(1)>>>(p, a, nblocks);
-    list_compute_kernel<R, 6, AVG><<<cb, 128, 0, s>>>(p, a, nblocks);
-    list_compute_kernel<R, 5, AVG><<<cb, 128, 0, fork.on(3)>>>(p, a, nblocks);
-    list_compute_kernel<R, 4, AVG><<<cb, 128, 0, s>>>(p, a, nblocks);
-    list_compute_kernel<R, 3, AVG><<<cb, 128, 0, fork.on(3)>>>(p, a, nblocks);
-    list_compute_kernel<R, 2, AVG><<<cb, 128, 0, fork.on(1)>>>(p, a, nblocks);
+    list_compute_kernel<R, 8, AVG><<<cb, 128, 0, fork.on(0)>>>(p, a, nblocks, together);
+    list_compute_kernel<R, 7, AVG><<<cb, 128, 0, fork.on(1)>>>(p, a, nblocks, together);
+    list_compute_kernel<R, 6, AVG><<<cb, 128, 0, s>>>(p, a, nblocks, together);
+    list_compute_kernel<R, 5, AVG><<<cb, 128, 0, fork.on(3)>>>(p, a, nblocks, together);
+    list_compute_kernel<R, 4, AVG><<<cb, 128, 0, s>>>(p, a, nblocks, together);
+    list_compute_kernel<R, 3, AVG><<<cb, 128, 0, fork.on(3)>>>(p, a, nblocks, together);
+    list_compute_kernel<R, 2, AVG><<<cb, 128, 0, fork.on(1)>>>(p, a, nblocks, together);
 }
 
 template <class R, int KS, int KL, int NS>
@@ -1259,8 +1270,9 @@ int launch_tiled_ns(const StepParams& p, const StepArrays& a, void* stream, Laun
     else
     {
         if (general_beside) gk<<<148 * 4, 128, wsm, fork.on(2)>>>(p, a);
-        if (a.avg_mask) launch_lists<R, true>(p, a, cb, nblocks, fork);
-        else launch_lists<R, false>(p, a, cb, nblocks, fork);
+        const bool together = info && info->worklist > (unsigned long long)p.n / kTogetherShare;
+        if (a.avg_mask) launch_lists<R, true>(p, a, cb, nblocks, fork, together);
+        else launch_lists<R, false>(p, a, cb, nblocks, fork, together);
     }
     if ((e = fork.join()) != cudaSuccess) return (int)e;
     if (info) info->kernels += p.aniso ? 4 : 10;
