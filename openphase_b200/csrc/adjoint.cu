@@ -82,6 +82,26 @@ __device__ __forceinline__ double force_slope(const StepParams& p, const StepArr
     return 1.0 - t * t;
 }
 
+// Whether all lanes that are here together have it: a warp whose lists mix grains at and below their
+// reference volume runs the general kinetics for all of them instead of both branches in turn.
+__device__ __forceinline__ bool warp_agrees(bool mine) { return __all_sync(__activemask(), mine); }
+
+// The worklist voxels of a thread, first and stride.  Each voxel is one long chain with branches of its own.
+// Up to 2400 of them get a warp each (56 x 60 x 50: adjoint step 0.66 ms, 0.78 in runs); more are dealt out
+// in runs of consecutive entries, neighbours whose chains and gathers are alike, as long as `warps` of them
+// hold the list and 32 at most (adjoint step, strided lanes -> runs, FP64: 96^3, 3.7 k voxels 3.84 -> 3.65 ms;
+// 48^3, 39 k 6.14 -> 5.18; 192^3, 24 k 10.7 -> 9.75).  32 blocks an SM instead of eight keep the end of a long
+// list short (96^3, 330 k: 68 -> 30 ms).
+struct WorkShare {
+    unsigned first, stride;
+};
+__device__ __forceinline__ WorkShare work_share(unsigned total, unsigned warps)
+{
+    const unsigned run = total <= 2400u ? 1u : min(32u, (total + warps - 1u) / warps), lane = threadIdx.x & 31u;
+    const unsigned warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    return {lane < run ? warp * run + lane : total, gridDim.x * (blockDim.x >> 5) * run};
+}
+
 // ---- tangent-linear step (FP64 form) --------------------------------------------------------------
 // Stages 2-5 of list_step<double> on dual numbers, operation by operation in the same order, so the
 // value parts are the forward's bit for bit and every decision is the forward's.
@@ -108,6 +128,7 @@ __device__ __forceinline__ int stages_dual(const StepParams& p, const StepArrays
     const double pref = p.pref_do;
     bool plain = p.tj_factor == 0.0;   // as in list_compute_kernel: one sum per field
     for (int k = 0; k < n; k++) plain = plain && a.vr[g[k]] == 1.0;
+    plain = warp_agrees(plain);
     if (plain)
     {
         for (int k = 0; k < n; k++) pos[k] = lap[k] + pref * val[k];
@@ -442,6 +463,9 @@ __global__ void __launch_bounds__(128) tlm_list_kernel(const __grid_constant__ S
     tlm_block_end(B, a, aa, eout, st);
 }
 
+// Below this length the tangent's worklist goes to strided lanes (48^3, 39 k voxels, step: 2.76 ms, in runs
+// 3.7); beyond, to runs (96^3, 330 k: 11.3 -> 6.6 with the votes of warp_agrees).
+constexpr unsigned kTangentScatter = 40000;
 template <int KS>
 __global__ void __launch_bounds__(64) tlm_worklist_kernel(const __grid_constant__ StepParams p, const StepArrays a,
                                                            const AdjArrays aa)
@@ -450,11 +474,15 @@ __global__ void __launch_bounds__(64) tlm_worklist_kernel(const __grid_constant_
     tlm_block_begin(B);
     const unsigned total = min(*a.slow_count, a.slow_cap);
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&a.counters[kCntGeneralLast], (unsigned long long)total);
-    const unsigned warps = gridDim.x * (blockDim.x >> 5);
-    const unsigned warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    WorkShare w = work_share(total, 600u);
+    if (total < kTangentScatter)   // one lane of each warp after the other
+    {
+        const unsigned warps = gridDim.x * (blockDim.x >> 5);
+        w = {(threadIdx.x & 31u) * warps + blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), 32u * warps};
+    }
     uint32_t st = 0;
     unsigned eout = 0;
-    for (unsigned i = (threadIdx.x & 31u) * warps + warp; i < total; i += 32u * warps)   // as the adjoint's worklist
+    for (unsigned i = w.first; i < total; i += w.stride)
     {
         const long long v = a.slow_list[i];
         const Neighbourhood nb(p, v);
@@ -673,6 +701,7 @@ __device__ __forceinline__ void adjoint_core(const StepParams& p, const StepArra
         vr[k] = a.vr[g[k]];
         plain = plain && vr[k] == 1.0;
     }
+    plain = warp_agrees(plain);
     double localN;
     if (p.consider_nucleus_volume)
     {
@@ -1105,12 +1134,9 @@ __global__ void __launch_bounds__(64) adjoint_worklist_kernel(const __grid_const
                                                                const AdjArrays aa)
 {
     constexpr int KL = KAdjList;
-    // Each voxel is one long chain with branches of its own: consecutive voxels go to different warps,
-    // so that a warp holds as few of them as there are warps for.
     const unsigned total = min(*a.slow_count, a.slow_cap);
-    const unsigned warps = gridDim.x * (blockDim.x >> 5);
-    const unsigned warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    for (unsigned i = (threadIdx.x & 31u) * warps + warp; i < total; i += 32u * warps)
+    const WorkShare w = work_share(total, 300u);
+    for (unsigned i = w.first; i < total; i += w.stride)
     {
         const long long v = a.slow_list[i];
         const Neighbourhood nb(p, v);
@@ -1280,15 +1306,16 @@ __global__ void lambda_init_kernel(long long N, const uint8_t* __restrict__ cnt,
 static unsigned grid_of(long long n, int t) { return (unsigned)((n + t - 1) / t); }
 
 int launch_tlm_step(const StepParams& p, const StepArrays& a, const AdjArrays& aa, int k_slots, int nblocks, void* stream,
-                    const SideStreams& side)
+                    const SideStreams& side, unsigned worklist)
 {
     const SideFork fork(&side, static_cast<cudaStream_t>(stream));
+    const int tangent_blocks = 148 * (worklist < kTangentScatter ? 8 : 32);
     bool known = true;
     switch (k_slots)
     {
-        case 8:  tlm_worklist_kernel<8><<<148 * 8, 64, 0, fork.on(0)>>>(p, a, aa); break;
-        case 12: tlm_worklist_kernel<12><<<148 * 8, 64, 0, fork.on(0)>>>(p, a, aa); break;
-        case 16: tlm_worklist_kernel<16><<<148 * 8, 64, 0, fork.on(0)>>>(p, a, aa); break;
+        case 8:  tlm_worklist_kernel<8><<<tangent_blocks, 64, 0, fork.on(0)>>>(p, a, aa); break;
+        case 12: tlm_worklist_kernel<12><<<tangent_blocks, 64, 0, fork.on(0)>>>(p, a, aa); break;
+        case 16: tlm_worklist_kernel<16><<<tangent_blocks, 64, 0, fork.on(0)>>>(p, a, aa); break;
         default: known = false; break;
     }
     tlm_list_kernel<8><<<148 * 8, 128, 0, fork.on(1)>>>(p, a, aa, nblocks);
@@ -1317,7 +1344,7 @@ static void adjoint_kernels(const StepParams& p, const StepArrays& a, const AdjA
 {
     const cudaStream_t s = fork.main;
     auto on = [&](int k) { return lists_beside ? fork.on(k) : s; };
-    adjoint_worklist_kernel<R, KS><<<148 * 8, 64, 0, fork.on(2)>>>(p, a, aa);
+    adjoint_worklist_kernel<R, KS><<<148 * 32, 64, 0, fork.on(2)>>>(p, a, aa);
     adjoint_list_kernel<R, 8><<<kAdjListBlocks, 128, 0, on(0)>>>(p, a, aa, nblocks);
     adjoint_list_kernel<R, 7><<<kAdjListBlocks, 128, 0, on(1)>>>(p, a, aa, nblocks);
     adjoint_list_kernel<R, 6><<<kAdjListBlocks, 128, 0, s>>>(p, a, aa, nblocks);

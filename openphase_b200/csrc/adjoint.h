@@ -34,7 +34,7 @@ struct AdjArrays {
 // classify kernel has run on the state (its work records, buckets and worklist in a; nblocks its
 // block count).
 int launch_tlm_step(const StepParams& p, const StepArrays& a, const AdjArrays& aa, int k_slots, int nblocks, void* stream,
-                    const SideStreams& side);
+                    const SideStreams& side, unsigned worklist);
 // Adjoint of one step: a.cnt_in/idx_in/val_in hold the state before the step, aa the state after it
 // and its adjoint; the classify kernel has just run on the state before the step (its work
 // records, buckets and worklist in a; nblocks its block count).  Writes the adjoint of the state

@@ -1872,7 +1872,7 @@ extern "C" uint32_t opgpu_tlm_step(opgpu_ctx* ctx, double dt, int32_t nsteps)
         const int nblocks = launch_classify_f64(sp, a, ctx->stream);
         if (nblocks < 0) return fail(ctx, OPGPU_E_CUDA, "opgpu_tlm_step: classify launch");
         // every stored entry of the new state gets its tangent
-        if (launch_tlm_step(sp, a, aa, ctx->K, nblocks, ctx->stream, ctx->side)) return fail(ctx, OPGPU_E_CUDA, "opgpu_tlm_step: launch");
+        if (launch_tlm_step(sp, a, aa, ctx->K, nblocks, ctx->stream, ctx->side, ctx->worklist)) return fail(ctx, OPGPU_E_CUDA, "opgpu_tlm_step: launch");
         grains_update_kernel<<<grid_for(ctx->G, 256), 256, 0, ctx->stream>>>(ctx->G, ctx->d_vol_acc, ctx->d_volume,
             ctx->d_maxvol, ctx->d_refvol, ctx->d_vr, ctx->d_exist, ctx->d_gstage, ctx->d_counters, 1);
         CK(cudaGetLastError());

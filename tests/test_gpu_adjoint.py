@@ -107,6 +107,24 @@ def test_general_kinetics_tangent_and_adjoint(name):
     assert R.adjoint_status == 0
 
 
+def test_tangent_steps_every_voxel_of_a_long_worklist():
+    """Small grains: a quarter of the voxels go to the general-path worklist, beyond the length where it is
+    dealt out in runs of neighbours.  The lists of more than 16 fields there overflow (reported); all other
+    voxels step as the forward does.  (A voxel left out would keep values of two steps before.)"""
+    case = Case(64, 64, 64, 152, seed=2, iwidth=6.0, dt=0.08, sigma=1.2, sigma_pairs=(0.8, 0.4), dg_scale=0.03,
+                name="long_worklist")
+    ctx, R, state, *_ = _setup(case=case, nsteps=1)
+    ctx.step(case.dt, 8)
+    ctx.checkpoint_save(0)
+    before = ctx.stats()["general_path_total"]
+    ctx.step(case.dt, 1)
+    assert ctx.stats()["general_path_total"] - before >= 40000
+    forward = ctx.download()
+    R.tangent(None, None, np.ones(case.ngrains))
+    r = compare_states(ctx.download(), forward, case.ngrains)
+    assert r["frac_over_1e4"] <= 0.02, r
+
+
 def _fd_check(h_rel, seed, case=CASE, nsteps=T, interval=None, precision="fp64"):
     """Central differences on 32 random parameters (12 sigma pairs, 12 mu pairs, 8 driving forces)
     of L = sum_g w_g V_g(T); L is summed on the host in a fixed order (deterministic)."""
