@@ -283,7 +283,8 @@ void*    opgpu_stream(opgpu_ctx* ctx);
  * zeroed and limited increments, snapped and erased fields) are those of the forward run and held
  * fixed; VolumeRatio is held fixed.  Both precisions record states; the adjoint arithmetic and the
  * gradient accumulation are FP64.  The tangent-linear model runs the FP64 form. */
-/* Reserve nslots device checkpoints (state plus grain records). */
+/* Reserve nslots device checkpoints (state plus grain records).  They stay reserved when opgpu_set_grains
+ * changes the number of grains, but hold no state then; a sweep begun before is begun anew. */
 uint32_t opgpu_checkpoint_reserve(opgpu_ctx* ctx, int32_t nslots);
 /* Copy the current state and grain records into / out of a checkpoint slot.  A slot that was reserved
  * but never saved (by opgpu_checkpoint_save or opgpu_step_save_input) holds no state: loading it or

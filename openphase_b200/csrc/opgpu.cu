@@ -403,6 +403,26 @@ void free_grains(opgpu_ctx* c)
     c->pair_energy_dirty = true;
 }
 
+// What was sized by another number of grains: the checkpoints' grain records (the slots then hold no
+// state) and the gradients and tangents of the parameters.  opgpu_checkpoint_reserve, ensure_adjoint and
+// ensure_tlm make them again.
+void drop_grain_sized(opgpu_ctx* c)
+{
+    for (auto& s : c->slots)
+    {
+        dfree(s.volume); dfree(s.maxvol); dfree(s.vr); dfree(s.exist); dfree(s.stage);
+        s.volume = s.maxvol = s.vr = nullptr;
+        s.exist = s.stage = nullptr;
+        s.saved = false;
+    }
+    for (double** p : {&c->d_gsig, &c->d_gmu, &c->d_gdg, &c->d_tsig, &c->d_tmu, &c->d_tdg, &c->d_tvol})
+    {
+        dfree(*p);
+        *p = nullptr;
+    }
+    c->adjoint_ready = c->tlm_ready = false;
+}
+
 // Tools::getDisorientationCubic (src/Tools.cpp:626-678): rotation angle 2*acos(max |c|) of
 // dQ = A * B.inverted() over the 24 component combinations c of the cubic group (Grimmer 1974),
 // with the reference's factors 0.707 and 0.5; quaternion product and inverse as
@@ -869,6 +889,7 @@ extern "C" uint32_t opgpu_set_grains(opgpu_ctx* ctx, int32_t ngrains, const int3
     if (!reserve_stage(ctx, G)) return fail(ctx, OPGPU_E_CUDA, "opgpu_set_grains: no pinned memory for the grain records");
     if (uint32_t r = make_side_streams(ctx)) return r;
     free_grains(ctx);
+    if (ctx->G != G) drop_grain_sized(ctx);
     ctx->G = G;
     ctx->sp.ngrains = G;
     CK(dalloc(&ctx->d_vr, G));
@@ -1619,6 +1640,18 @@ uint32_t copy_state(opgpu_ctx* ctx, uint8_t* dc, int16_t* di, void* dv, const ui
     return OPGPU_OK;
 }
 
+// The grain records of a slot (a slot has none after opgpu_set_grains with another number of grains).
+uint32_t reserve_records(opgpu_ctx* ctx, opgpu_ctx::Slot& s)
+{
+    const size_t G = (size_t)ctx->G;
+    if (!s.volume) CK(dalloc(&s.volume, G));
+    if (!s.maxvol) CK(dalloc(&s.maxvol, G));
+    if (!s.vr) CK(dalloc(&s.vr, G));
+    if (!s.exist) CK(dalloc(&s.exist, G));
+    if (!s.stage) CK(dalloc(&s.stage, G));
+    return OPGPU_OK;
+}
+
 uint32_t copy_grains(opgpu_ctx* ctx, double* vol, double* mx, double* vr, int8_t* ex, int8_t* stg,
                      const double* svol, const double* smx, const double* svr, const int8_t* sex, const int8_t* sstg)
 {
@@ -1644,14 +1677,15 @@ uint32_t ensure_adjoint(opgpu_ctx* ctx)
         return fail(ctx, OPGPU_E_INVALID, "the adjoint and tangent-linear steps do not support driving-force averaging");
     if (ctx->adjoint_ready) return OPGPU_OK;
     const size_t N = (size_t)ctx->n, K = (size_t)ctx->K, G = (size_t)ctx->G;
-    for (int b = 0; b < 2; b++) CK(dalloc(&ctx->d_lam[b], N * K));
-    CK(dalloc(&ctx->d_lam_local, N * K));
-    CK(dalloc(&ctx->d_lcnt, N));
-    CK(dalloc(&ctx->d_lidx, N * KAdjList));
-    CK(dalloc(&ctx->d_llam, N * KAdjList));
-    CK(dalloc(&ctx->d_gsig, G * G));
-    CK(dalloc(&ctx->d_gmu, G * G));
-    CK(dalloc(&ctx->d_gdg, G));
+    auto make = [](auto** p, size_t count) { return *p ? cudaSuccess : dalloc(p, count); };
+    for (int b = 0; b < 2; b++) CK(make(&ctx->d_lam[b], N * K));
+    CK(make(&ctx->d_lam_local, N * K));
+    CK(make(&ctx->d_lcnt, N));
+    CK(make(&ctx->d_lidx, N * KAdjList));
+    CK(make(&ctx->d_llam, N * KAdjList));
+    CK(make(&ctx->d_gsig, G * G));
+    CK(make(&ctx->d_gmu, G * G));
+    CK(make(&ctx->d_gdg, G));
     ctx->adjoint_ready = true;
     return OPGPU_OK;
 }
@@ -1662,11 +1696,12 @@ uint32_t ensure_tlm(opgpu_ctx* ctx)
         return fail(ctx, OPGPU_E_INVALID, "the adjoint and tangent-linear steps do not support driving-force averaging");
     if (ctx->tlm_ready) return OPGPU_OK;
     const size_t N = (size_t)ctx->n, K = (size_t)ctx->K, G = (size_t)ctx->G;
-    for (int b = 0; b < 2; b++) CK(dalloc(&ctx->d_dphi[b], N * K));
-    CK(dalloc(&ctx->d_tsig, G * G));
-    CK(dalloc(&ctx->d_tmu, G * G));
-    CK(dalloc(&ctx->d_tdg, G));
-    CK(dalloc(&ctx->d_tvol, G));
+    auto make = [](auto** p, size_t count) { return *p ? cudaSuccess : dalloc(p, count); };
+    for (int b = 0; b < 2; b++) CK(make(&ctx->d_dphi[b], N * K));
+    CK(make(&ctx->d_tsig, G * G));
+    CK(make(&ctx->d_tmu, G * G));
+    CK(make(&ctx->d_tdg, G));
+    CK(make(&ctx->d_tvol, G));
     ctx->tlm_ready = true;
     return OPGPU_OK;
 }
@@ -1690,17 +1725,17 @@ extern "C" uint32_t opgpu_checkpoint_reserve(opgpu_ctx* ctx, int32_t nslots)
 {
     if (uint32_t r = require(ctx, ctx && ctx->G > 0, "opgpu_checkpoint_reserve: set the grains first")) return r;
     if (nslots < 0 || nslots > 4096) return fail(ctx, OPGPU_E_INVALID, "opgpu_checkpoint_reserve: 0..4096 slots");
-    const size_t N = (size_t)ctx->n, K = (size_t)ctx->K, G = (size_t)ctx->G;
+    const size_t N = (size_t)ctx->n, K = (size_t)ctx->K;
     while ((int)ctx->slots.size() < nslots)
     {
         opgpu_ctx::Slot s;
         CK(dalloc(&s.cnt, N));
         CK(dalloc(&s.idx, N * K));
         CK(cudaMalloc(&s.val, N * K * ctx->rsz + 16));
-        CK(dalloc(&s.volume, G)); CK(dalloc(&s.maxvol, G)); CK(dalloc(&s.vr, G));
-        CK(dalloc(&s.exist, G)); CK(dalloc(&s.stage, G));
         ctx->slots.push_back(s);
     }
+    for (auto& s : ctx->slots)
+        if (uint32_t r = reserve_records(ctx, s)) return r;
     return OPGPU_OK;
 }
 
@@ -1710,6 +1745,7 @@ extern "C" uint32_t opgpu_checkpoint_save(opgpu_ctx* ctx, int32_t slot)
     if (slot < 0 || slot >= (int)ctx->slots.size()) return fail(ctx, OPGPU_E_INVALID, "opgpu_checkpoint_save: no such slot");
     auto& s = ctx->slots[slot];
     s.saved = false;
+    if (uint32_t r = reserve_records(ctx, s)) return r;
     if (uint32_t r = copy_state(ctx, s.cnt, s.idx, s.val, ctx->cnt[ctx->cur], ctx->idx[ctx->cur], ctx->val[ctx->cur])) return r;
     if (uint32_t r = copy_grains(ctx, s.volume, s.maxvol, s.vr, s.exist, s.stage, ctx->d_volume, ctx->d_maxvol, ctx->d_vr,
                                  ctx->d_exist, ctx->d_gstage)) return r;
@@ -1724,6 +1760,7 @@ extern "C" uint32_t opgpu_step_save_input(opgpu_ctx* ctx, double dt, int32_t slo
     auto& s = ctx->slots[slot];
     // the grain records are updated in place by the step: copy them first (G values)
     s.saved = false;
+    if (uint32_t r = reserve_records(ctx, s)) return r;
     if (uint32_t r = copy_grains(ctx, s.volume, s.maxvol, s.vr, s.exist, s.stage, ctx->d_volume, ctx->d_maxvol,
                                  ctx->d_vr, ctx->d_exist, ctx->d_gstage)) return r;
     const int in = ctx->cur;

@@ -95,3 +95,33 @@ def test_slots_that_were_never_saved_are_refused(precision):
     R.forward()
     R.backward(w)
     assert R.adjoint_status == 0
+
+
+@pytest.mark.parametrize("grains", [(6, 40), (40, 6)])
+def test_slots_and_sweeps_follow_the_number_of_grains(grains):
+    """Checkpoints and adjoint buffers of a context that takes another number of grains: the slots hold no
+    state, and forward and backward give what a new context gives."""
+    def rollout(ctx, case):
+        G = case.ngrains
+        ctx.set_pair_table(np.ones((G, G)), np.ones((G, G)))
+        R = Rollout(ctx, case.dt, 6)
+        volume = R.forward()
+        grads = R.backward(np.arange(G) - 0.5 * G)
+        dv = R.tangent(None, None, np.arange(G) * 0.1)
+        return [volume, *grads, dv]
+
+    first, second = (Case(22, 20, 18, G, seed=G, iwidth=4.0, dt=0.08, dg_scale=0.05, name="regrain") for G in grains)
+    ctx = Context.from_case(first, precision="fp64", k_slots=16)
+    rollout(ctx, first)
+    ctx.set_grains(second.ngrains)
+    ctx.set_driving_force(second.driving_force())
+    ctx.upload(*second.initial_state())
+    ctx.finalize_initialization()
+    for call in (lambda: ctx.checkpoint_load(0), lambda: ctx.adjoint_step(1, second.dt), lambda: ctx.tlm_step(second.dt)):
+        with pytest.raises(OpgpuError) as e:
+            call()
+        assert e.value.code & E_STATE
+    got = rollout(ctx, second)
+    expected = rollout(Context.from_case(second, precision="fp64", k_slots=16), second)
+    for a, b in zip(got, expected):   # up to the order of the atomic sums
+        assert np.allclose(a, b, rtol=1e-9, atol=1e-9 * np.abs(b).max())
