@@ -27,7 +27,6 @@ enum : uint32_t {
     kStLimiterCap = 1u << 4,
     kStNonFinite = 1u << 5,
     kStAdjointMismatch = 1u << 6,   // the recomputed step does not reproduce the stored next state
-    kStAverageSkipped = 1u << 7,    // reserved: averaging has no per-pair storage to run out of
 };
 
 // Driving-force averaging (average.cu): one bit per pair of stored fields of every interface voxel,
@@ -164,7 +163,8 @@ constexpr int kTileRows = 8;   // one thread each
 // planes times waves, plus a third of a wave for blocks over bulk and over interfaces that differ in
 // length; the shortest wins.  Measured, classify in us (chunk): FP64 64^3 81 (2) 62 (5); 96^3 181 (5) 151
 // (8) 140 (16); 128^3 318 (13) 345 (16) 372 (43); 160^3 566 (15) 577 (20); FP32 150x97x203, 7-point 376
-// (15) 365 (21) 341 (38): the estimate's order each time.  slice = voxels one block can append to a
+// (15) 365 (21) 341 (38).  The estimate's choice is the fastest measured one each time (13 at 128^3, where
+// it ranks 43 before 16, the other way round than measured).  slice = voxels one block can append to a
 // bucket.
 inline void tiled_geometry(int nx, int ny, int nz, int real_size, int* xchunk, int* gz, int* gy, int* gx)
 {

@@ -8,7 +8,8 @@
 //   every ring plane is held twice: per record its slots in entry order with a slot bitmask, and as
 //   dense per-slot value planes dense[slot][plane][record] (zero where the grain is absent).  For
 //   each voxel of the centre plane one thread
-//     - derives the flag from the 27 neighbour counts and copies bulk voxels to the output;
+//     - derives the flag from its count and the "several fields" bits of the 27 records' words, and
+//       copies bulk voxels to the output;
 //     - discovers the candidate fields with bitmask operations, in the reference's order (own
 //       fields, then new grains in stencil order and neighbour-list order);
 //     - sums every field's Laplacian from the dense planes (27 loads and multiply-adds in stencil
@@ -18,8 +19,9 @@
 // compute (list_compute_kernel<N>)
 //   One kernel per list length N = 2..kListCap over all the slices' entries of that length (a
 //   small scan kernel turns the per-slice counts into offsets), split evenly over the CUDA blocks:
-//   fully unrolled, register-only pair kinetics, driving force, projection, merge and finalize
-//   (the operation order of list_step), new record written to the output state.
+//   fully unrolled pair kinetics, driving force, projection, merge and finalize (the operation order
+//   of list_step; from N = 5 on some of the arrays lie in local memory), new record written to the
+//   output state.
 // Lists longer than kListCap and voxels next to a grain without a window slot go to the general-path
 // worklist, processed one warp per voxel (warp_step.cuh).
 #pragma once
@@ -38,8 +40,8 @@ struct WindowSlots {
 constexpr int kSlotMap = 512;        // grain -> slot map entries
 constexpr int kTileVolSlots = 512;      // grain-volume hash of the compute kernels
 // Entries per record the plane loader keeps in registers.  FP32 has 96 registers at five blocks per SM
-// and spills with six (256^3, classify: 1894 us with six, 1760 with four); FP64 has 160 at three blocks,
-// and the records beyond four cost more (2060 with six, 2178 with four).
+// and spills with six (256^3, classify: 1894 us with six, 1760 with four); FP64 has room for 160 at three
+// blocks (it takes 135 to 144), and the records beyond four cost more (2060 with six, 2178 with four).
 template <class R>
 struct KeepEntries {
     static constexpr int value = sizeof(R) == 8 ? 6 : 4;
