@@ -344,18 +344,18 @@ __global__ void __launch_bounds__(128) df_tiles_kernel(const __grid_constant__ S
                                                         const double* __restrict__ vr)
 {
     constexpr unsigned kParts = kReachX * kReachY * kReachZ / 32;
-    const unsigned items = aa.tiles[0] * kParts, lane = threadIdx.x & 31u;
-    while (true)
+    const unsigned items = aa.tiles[0] * kParts, lane = threadIdx.x & 31u, warps = gridDim.x * (blockDim.x >> 5);
+    // a warp's first item is its own number (no tile listed: nothing is fetched), the next ones are counted
+    for (unsigned item = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); item < items;)
     {
-        unsigned item = lane == 0 ? atomicAdd(&aa.tiles[1], 1u) : 0u;
-        item = __shfl_sync(0xffffffffu, item, 0);
-        if (item >= items) return;
         const unsigned tile = aa.tiles[2u + item / kParts], i = (item % kParts) * 32u + lane;
         const int x = (int)(tile / (gx * gy) * kReachX + i / (kReachZ * kReachY));
         const int y = (int)(tile / gx % gy * kReachY + i / kReachZ % kReachY);
         const int z = (int)(tile % gx * kReachZ + i % kReachZ);
         if (x < p.nx && y < p.ny && z < p.nz) search_sphere<R>(p, aa, cnt, idx, val, vr, x, y, z);
         __syncwarp();
+        item = lane == 0 ? warps + atomicAdd(&aa.tiles[1], 1u) : 0u;
+        item = __shfl_sync(0xffffffffu, item, 0);
     }
 }
 
@@ -369,7 +369,7 @@ int launch_average_of(const StepParams& p, const AvgArrays& aa, const uint8_t* c
     if (aa.range <= kReachRange && tiles.y <= 65535u && tiles.z <= 65535u)
     {
         df_reach_kernel<R><<<tiles, 256, 0, s>>>(p, aa, cnt, idx, val, vr);
-        df_tiles_kernel<R><<<148 * 16, 128, 0, s>>>(p, aa, tiles.y, tiles.x, cnt, idx, val, vr);
+        df_tiles_kernel<R><<<148 * 8, 128, 0, s>>>(p, aa, tiles.y, tiles.x, cnt, idx, val, vr);
         *kernels += 3;
     }
     else
