@@ -90,8 +90,10 @@ __device__ __forceinline__ bool warp_agrees(bool mine) { return __all_sync(__act
 // Up to 2400 of them get a warp each (56 x 60 x 50: adjoint step 0.66 ms, 0.78 in runs); more are dealt out
 // in runs of consecutive entries, neighbours whose chains and gathers are alike, as long as `warps` of them
 // hold the list and 32 at most (adjoint step, strided lanes -> runs, FP64: 96^3, 3.7 k voxels 3.84 -> 3.65 ms;
-// 48^3, 39 k 6.14 -> 5.18; 192^3, 24 k 10.7 -> 9.75).  32 blocks an SM instead of eight keep the end of a long
-// list short (96^3, 330 k: 68 -> 30 ms).
+// 48^3, 39 k 6.14 -> 5.18; 192^3, 24 k 10.7 -> 9.75).  Eight blocks an SM hold a short list's runs; 32 keep the
+// end of a long list short (96^3, 330 k: 68 -> 30 ms).  The launch goes by the length the host knows.
+constexpr unsigned kLongWorklist = 40000;
+inline unsigned worklist_blocks(unsigned worklist) { return 148u * (worklist < kLongWorklist ? 8u : 32u); }
 struct WorkShare {
     unsigned first, stride;
 };
@@ -463,9 +465,8 @@ __global__ void __launch_bounds__(128) tlm_list_kernel(const __grid_constant__ S
     tlm_block_end(B, a, aa, eout, st);
 }
 
-// Below this length the tangent's worklist goes to strided lanes (48^3, 39 k voxels, step: 2.76 ms, in runs
-// 3.7); beyond, to runs (96^3, 330 k: 11.3 -> 6.6 with the votes of warp_agrees).
-constexpr unsigned kTangentScatter = 40000;
+// A worklist that is not long goes to strided lanes here (48^3, 39 k voxels, step: 2.76 ms, in runs 3.7); a
+// long one to runs (96^3, 330 k: 11.3 -> 6.6 with the votes of warp_agrees).
 template <int KS>
 __global__ void __launch_bounds__(64) tlm_worklist_kernel(const __grid_constant__ StepParams p, const StepArrays a,
                                                            const AdjArrays aa)
@@ -475,7 +476,7 @@ __global__ void __launch_bounds__(64) tlm_worklist_kernel(const __grid_constant_
     const unsigned total = min(*a.slow_count, a.slow_cap);
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&a.counters[kCntGeneralLast], (unsigned long long)total);
     WorkShare w = work_share(total, 600u);
-    if (total < kTangentScatter)   // one lane of each warp after the other
+    if (total < kLongWorklist)   // one lane of each warp after the other
     {
         const unsigned warps = gridDim.x * (blockDim.x >> 5);
         w = {(threadIdx.x & 31u) * warps + blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), 32u * warps};
@@ -701,7 +702,6 @@ __device__ __forceinline__ void adjoint_core(const StepParams& p, const StepArra
         vr[k] = a.vr[g[k]];
         plain = plain && vr[k] == 1.0;
     }
-    plain = warp_agrees(plain);
     double localN;
     if (p.consider_nucleus_volume)
     {
@@ -1309,13 +1309,13 @@ int launch_tlm_step(const StepParams& p, const StepArrays& a, const AdjArrays& a
                     const SideStreams& side, unsigned worklist)
 {
     const SideFork fork(&side, static_cast<cudaStream_t>(stream));
-    const int tangent_blocks = 148 * (worklist < kTangentScatter ? 8 : 32);
+    const unsigned blocks = worklist_blocks(worklist);
     bool known = true;
     switch (k_slots)
     {
-        case 8:  tlm_worklist_kernel<8><<<tangent_blocks, 64, 0, fork.on(0)>>>(p, a, aa); break;
-        case 12: tlm_worklist_kernel<12><<<tangent_blocks, 64, 0, fork.on(0)>>>(p, a, aa); break;
-        case 16: tlm_worklist_kernel<16><<<tangent_blocks, 64, 0, fork.on(0)>>>(p, a, aa); break;
+        case 8:  tlm_worklist_kernel<8><<<blocks, 64, 0, fork.on(0)>>>(p, a, aa); break;
+        case 12: tlm_worklist_kernel<12><<<blocks, 64, 0, fork.on(0)>>>(p, a, aa); break;
+        case 16: tlm_worklist_kernel<16><<<blocks, 64, 0, fork.on(0)>>>(p, a, aa); break;
         default: known = false; break;
     }
     tlm_list_kernel<8><<<148 * 8, 128, 0, fork.on(1)>>>(p, a, aa, nblocks);
@@ -1340,11 +1340,11 @@ constexpr int kAdjListBlocks = 148 * 32;   // blocks of each per-length adjoint 
 // beside each other there; with `lists_beside` false only the worklist kernel has another stream.
 template <class R, int KS>
 static void adjoint_kernels(const StepParams& p, const StepArrays& a, const AdjArrays& aa, int nblocks,
-                            const SideFork& fork, bool lists_beside)
+                            const SideFork& fork, bool lists_beside, unsigned blocks)
 {
     const cudaStream_t s = fork.main;
     auto on = [&](int k) { return lists_beside ? fork.on(k) : s; };
-    adjoint_worklist_kernel<R, KS><<<148 * 32, 64, 0, fork.on(2)>>>(p, a, aa);
+    adjoint_worklist_kernel<R, KS><<<blocks, 64, 0, fork.on(2)>>>(p, a, aa);
     adjoint_list_kernel<R, 8><<<kAdjListBlocks, 128, 0, on(0)>>>(p, a, aa, nblocks);
     adjoint_list_kernel<R, 7><<<kAdjListBlocks, 128, 0, on(1)>>>(p, a, aa, nblocks);
     adjoint_list_kernel<R, 6><<<kAdjListBlocks, 128, 0, s>>>(p, a, aa, nblocks);
@@ -1361,15 +1361,16 @@ int launch_adjoint_step(const StepParams& p, const StepArrays& a, const AdjArray
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const SideFork fork(worklist < kListsBeside ? &side : nullptr, s);
     const bool beside = worklist < kAdjointListsBeside;
+    const unsigned blocks = worklist_blocks(worklist);
     bool known = true;
     switch (k_slots * 2 + (fp32 ? 1 : 0))
     {
-        case 16: adjoint_kernels<double, 8>(p, a, aa, nblocks, fork, beside); break;
-        case 17: adjoint_kernels<float, 8>(p, a, aa, nblocks, fork, beside); break;
-        case 24: adjoint_kernels<double, 12>(p, a, aa, nblocks, fork, beside); break;
-        case 25: adjoint_kernels<float, 12>(p, a, aa, nblocks, fork, beside); break;
-        case 32: adjoint_kernels<double, 16>(p, a, aa, nblocks, fork, beside); break;
-        case 33: adjoint_kernels<float, 16>(p, a, aa, nblocks, fork, beside); break;
+        case 16: adjoint_kernels<double, 8>(p, a, aa, nblocks, fork, beside, blocks); break;
+        case 17: adjoint_kernels<float, 8>(p, a, aa, nblocks, fork, beside, blocks); break;
+        case 24: adjoint_kernels<double, 12>(p, a, aa, nblocks, fork, beside, blocks); break;
+        case 25: adjoint_kernels<float, 12>(p, a, aa, nblocks, fork, beside, blocks); break;
+        case 32: adjoint_kernels<double, 16>(p, a, aa, nblocks, fork, beside, blocks); break;
+        case 33: adjoint_kernels<float, 16>(p, a, aa, nblocks, fork, beside, blocks); break;
         default: known = false; break;
     }
     const cudaError_t e = fork.join();
